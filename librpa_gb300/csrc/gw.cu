@@ -18,8 +18,8 @@
 //
 // The four LibRI labels of cal_Hs / cal_Sigmas sum to one closed form,
 //   H_pq = sum_{a,b,r,s} U[a,p,r] W[a,b] U[b,q,s] D[r,s],   U[a,p,r] = C_a[p,r] + C_a[r,p],
-// which runs here as three FP64 GEMMs over dense operands: Y = U D ([(a,p), s]), Z = W U
-// ([a, (q,s)]) and H = Y' Z' over (a, s).  The dense U holds N_abf n_ao^2 values, which bounds
+// which runs here as three FP64 GEMMs over dense operands, for the rows p of one cell: Y = U D
+// ([(a,p), s]), Yw = W Y ([b, (p,s)]) and H = Yw U over (b, s).  The dense U holds N_abf n_ao^2 values, which bounds
 // this formulation to cells of a few hundred orbitals; larger cells need the atom-pair-sparse
 // form of the χ0 contraction.
 #include <algorithm>
@@ -58,32 +58,6 @@ __global__ void k_gamma_dm(const cuDoubleComplex *__restrict__ psi, const double
         acc += s[n] * (a.x * b.x + a.y * b.y);
     }
     G[t] = sgn * acc;
-}
-
-// Yt[p][(a, s)] = Y[(a, p), s]
-__global__ void k_perm_y(const double *__restrict__ Y, int N, int nao, double *__restrict__ Yt)
-{
-    const long long n = static_cast<long long>(N) * nao * nao;
-    for (long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; t < n;
-         t += static_cast<long long>(gridDim.x) * blockDim.x)
-    {
-        const long long a = t / (static_cast<long long>(nao) * nao);
-        const int p = static_cast<int>((t / nao) % nao), s = static_cast<int>(t % nao);
-        Yt[(static_cast<long long>(p) * N + a) * nao + s] = Y[t];
-    }
-}
-
-// Zt[(a, s)][q] = Z[a][(q, s)]
-__global__ void k_perm_z(const double *__restrict__ Z, int N, int nao, double *__restrict__ Zt)
-{
-    const long long n = static_cast<long long>(N) * nao * nao;
-    for (long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; t < n;
-         t += static_cast<long long>(gridDim.x) * blockDim.x)
-    {
-        const long long a = t / (static_cast<long long>(nao) * nao);
-        const int q = static_cast<int>((t / nao) % nao), s = static_cast<int>(t % nao);
-        Zt[(a * nao + s) * nao + q] = Z[t];
-    }
 }
 
 // In place: A <- I - A (batch of N x N)
@@ -271,9 +245,9 @@ __global__ void k_to_super(const double *__restrict__ src, long long cstride, in
     }
 }
 
-// Sig[w][c][K][L] += cw[w] (S+ + S-)/2 + i sw[w] (S+ - S-)/2 with S(R_c)_KL the supercell row block
-// of the cell R = 0 (row cell c0), column block c.
-__global__ void k_sigma_rows(const double *__restrict__ Sp, const double *__restrict__ Sm, int c0, int nc, int n,
+// Sig[w][c][K][L] += cw[w] (S+ + S-)/2 + i sw[w] (S+ - S-)/2 with S(R_c)_KL the home rows K (the cell
+// R = 0), column block c.
+__global__ void k_sigma_rows(const double *__restrict__ Sp, const double *__restrict__ Sm, int nc, int n,
                              const double *__restrict__ cw, const double *__restrict__ sw, int nw,
                              cuDoubleComplex *__restrict__ Sig)
 {
@@ -285,7 +259,7 @@ __global__ void k_sigma_rows(const double *__restrict__ Sp, const double *__rest
         const long long e = t % per;
         const int c = static_cast<int>(e / (static_cast<long long>(n) * n));
         const int K = static_cast<int>((e / n) % n), L = static_cast<int>(e % n);
-        const long long src = (static_cast<long long>(c0) * n + K) * ns + static_cast<long long>(c) * n + L;
+        const long long src = static_cast<long long>(K) * ns + static_cast<long long>(c) * n + L;
         const double cp = 0.5 * (Sp[src] + Sm[src]), sp = 0.5 * (Sp[src] - Sm[src]);
         cuDoubleComplex o = Sig[t];
         o.x += cw[w] * cp;
@@ -712,36 +686,139 @@ std::vector<double> dmat_r(const Dataset &ds, int s, const GammaSetup &gs)
     return DR;
 }
 
-// H[p][q] = sum U[a,p,r] W[a,b] U[b,q,s] D[r,s] for each of nd matrices D (nd <= 2); Z = W U is
-// formed once.  Work buffers: Y, Yt, Z, Zt.
+// Home rows of U: Uh[(a, p)][r] = U[a][c0 naoc + p][r] for the NAOs p of the cell R = 0.
+__global__ void k_home_rows(const double *__restrict__ U, int N, int nao, int naoc, int p0, double *__restrict__ Uh)
+{
+    const long long row = static_cast<long long>(naoc) * nao, n = static_cast<long long>(N) * row;
+    for (long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; t < n;
+         t += static_cast<long long>(gridDim.x) * blockDim.x)
+        Uh[t] = U[(t / row) * nao * nao + static_cast<long long>(p0) * nao + t % row];
+}
+
+// Partial products of the last step of the closed form, a short and wide output over a K axis (b, s)
+// that is N n_ao long:
+//   P[z][p][q] = sum_{k in part} Yw[d][b][p][s] U[b][s][q],   k = b n_ao + s, z = d nsplit + part.
+// Bound: the FP64 pipe (2 FMAs per clock per SM).  One CTA per output tile would run one SM or a few
+// for the whole product (2-atom fcc cell on 2x2x2 k: 16 CTAs with K = 133k, 0.12 s), so K is cut into
+// parts that fill the chip; the parts are summed in order by k_sum_parts, which keeps the result
+// independent of the schedule.  TM = 32 serves outputs of at most 32 rows without padding to 64.
+constexpr int HN = 64, HK = 16;
+
+template <int TM>
+__global__ void __launch_bounds__(256) k_hs_last(const double *__restrict__ Yw, const double *__restrict__ U, int N,
+                                                 int nao, int naoc, int nsplit, long long kpart, double *__restrict__ P)
+{
+    constexpr int RM = TM / 16;
+    __shared__ double As[HK][TM + 1];
+    __shared__ double Bs[HK][HN];
+    const int d = blockIdx.z / nsplit, part = blockIdx.z % nsplit;
+    const long long K = static_cast<long long>(N) * nao;
+    const long long k0 = part * kpart, k1 = min(K, k0 + kpart);
+    const double *Y = Yw + static_cast<long long>(d) * N * naoc * nao;
+    const int p0 = blockIdx.y * TM, q0 = blockIdx.x * HN;
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    double acc[RM][4] = {};
+    for (long long kb = k0; kb < k1; kb += HK)
+    {
+        for (int t = threadIdx.x; t < TM * HK; t += 256)
+        {
+            const int r = t / HK, kk = t % HK;
+            const long long k = kb + kk;
+            const long long b = k / nao, s = k % nao;
+            As[kk][r] = (k < k1 && p0 + r < naoc) ? Y[(b * naoc + p0 + r) * nao + s] : 0.0;
+        }
+        for (int t = threadIdx.x; t < HK * HN; t += 256)
+        {
+            const int kk = t / HN, c = t % HN;
+            const long long k = kb + kk;
+            Bs[kk][c] = (k < k1 && q0 + c < nao) ? U[k * nao + q0 + c] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < HK; ++kk)
+        {
+            double x[RM], y[4];
+#pragma unroll
+            for (int i = 0; i < RM; ++i) x[i] = As[kk][ty + 16 * i];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) y[j] = Bs[kk][tx + 16 * j];
+#pragma unroll
+            for (int i = 0; i < RM; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fma(x[i], y[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+    double *o = P + static_cast<long long>(blockIdx.z) * naoc * nao;
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            const int p = p0 + ty + 16 * i, q = q0 + tx + 16 * j;
+            if (p < naoc && q < nao) o[static_cast<long long>(p) * nao + q] = acc[i][j];
+        }
+}
+
+// H[d][e] = sum over the parts of P[d][part][e], in order
+__global__ void k_sum_parts(const double *__restrict__ P, long long n, int nsplit, double *__restrict__ H)
+{
+    const double *Pd = P + static_cast<long long>(blockIdx.y) * nsplit * n;
+    for (long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
+         e += static_cast<long long>(gridDim.x) * blockDim.x)
+    {
+        double acc = 0.0;
+        for (int k = 0; k < nsplit; ++k) acc += Pd[k * n + e];
+        H[blockIdx.y * n + e] = acc;
+    }
+}
+
+// H[d][p][q] = sum U[a,p,r] W[a,b] U[b,q,s] D[d][r,s] for the NAOs p of the cell R = 0 and every
+// supercell NAO q: the rows both callers read (every other row block is a translation of this one).
+// Y = U D on those rows, Yw = W Y, and H = Yw U over (b, s); with the row restriction every product
+// is n_cells smaller than on the whole supercell, which is why W multiplies Y here and not U.
 struct HsWork
 {
-    DevBuf<double> Y, Yt, Z, Zt;
+    DevBuf<double> Uh, Y, Yw, P;
 };
 
-void hs_closed_form(const GammaSetup &gs, const double *W, const double *const *D, int nd, double *const *H,
-                    HsWork &wk, cudaStream_t st)
+void hs_closed_form(const GammaSetup &gs, const double *W, const double *D, int nd, double *H, HsWork &wk, cudaStream_t st)
 {
-    const int N = gs.N, nao = gs.nao;
-    const long long nn = static_cast<long long>(nao) * nao, big = static_cast<long long>(N) * nn;
-    if (wk.Y.size() < static_cast<size_t>(big))
+    const int N = gs.N, nao = gs.nao, naoc = gs.naoc;
+    const long long nn = static_cast<long long>(nao) * nao, home = static_cast<long long>(N) * naoc * nao,
+                    hn = static_cast<long long>(naoc) * nao;
+    if (gs.nc > 1 && wk.Uh.size() == 0)
     {
-        wk.Y.alloc(big);
-        wk.Yt.alloc(big);
-        wk.Z.alloc(big);
-        wk.Zt.alloc(big);
-    }
-    launch_dgemm(N, static_cast<int>(nn), N, W, N, 0, gs.U.get(), nn, 0, wk.Z.get(), nn, 0, 1, 1.0, 0.0, st);
-    k_perm_z<<<grid_for(big), 256, 0, st>>>(wk.Z.get(), N, nao, wk.Zt.get());
-    GB_LAUNCH_CHECK();
-    for (int d = 0; d < nd; ++d)
-    {
-        launch_dgemm(N * nao, nao, nao, gs.U.get(), nao, 0, D[d], nao, 0, wk.Y.get(), nao, 0, 1, 1.0, 0.0, st);
-        k_perm_y<<<grid_for(big), 256, 0, st>>>(wk.Y.get(), N, nao, wk.Yt.get());
+        wk.Uh.alloc(home);
+        k_home_rows<<<grid_for(home), 256, 0, st>>>(gs.U.get(), N, nao, naoc, gs.c0 * naoc, wk.Uh.get());
         GB_LAUNCH_CHECK();
-        launch_dgemm(nao, nao, static_cast<int>(static_cast<long long>(N) * nao), wk.Yt.get(), static_cast<long long>(N) * nao,
-                     0, wk.Zt.get(), nao, 0, H[d], nao, 0, 1, 1.0, 0.0, st);
     }
+    if (wk.Y.size() < static_cast<size_t>(nd * home))
+    {
+        wk.Y.alloc(nd * home);
+        wk.Yw.alloc(nd * home);
+    }
+    const double *Uh = gs.nc > 1 ? wk.Uh.get() : gs.U.get();
+    launch_dgemm(N * naoc, nao, nao, Uh, nao, 0, D, nao, nn, wk.Y.get(), nao, home, nd, 1.0, 0.0, st);
+    launch_dgemm(N, static_cast<int>(hn), N, W, N, 0, wk.Y.get(), hn, home, wk.Yw.get(), hn, home, nd, 1.0, 0.0, st);
+    // parts of K: four CTAs per SM (the pipe is busy with one; the others cover its loads and the tail),
+    // at least 128 of K each
+    const bool narrow = naoc <= 32;
+    const long long K = static_cast<long long>(N) * nao, tiles = static_cast<long long>((nao + HN - 1) / HN) *
+                                                                 (narrow ? 1 : (naoc + 63) / 64) * nd;
+    const int nsplit = static_cast<int>(std::max<long long>(1, std::min<long long>((4 * 152 + tiles - 1) / tiles, K / 128)));
+    const long long kpart = ((K + nsplit - 1) / nsplit + HK - 1) / HK * HK;
+    if (wk.P.size() < static_cast<size_t>(nd) * nsplit * hn) wk.P.alloc(static_cast<size_t>(nd) * nsplit * hn);
+    const dim3 grid(static_cast<unsigned>((nao + HN - 1) / HN), static_cast<unsigned>(narrow ? 1 : (naoc + 63) / 64),
+                    static_cast<unsigned>(nd * nsplit));
+    if (narrow)
+        k_hs_last<32><<<grid, 256, 0, st>>>(wk.Yw.get(), gs.U.get(), N, nao, naoc, nsplit, kpart, wk.P.get());
+    else
+        k_hs_last<64><<<grid, 256, 0, st>>>(wk.Yw.get(), gs.U.get(), N, nao, naoc, nsplit, kpart, wk.P.get());
+    GB_LAUNCH_CHECK();
+    k_sum_parts<<<dim3(static_cast<unsigned>(std::min<long long>((hn + 255) / 256, 152LL * 8)), nd), 256, 0, st>>>(
+        wk.P.get(), hn, nsplit, H);
+    GB_LAUNCH_CHECK();
 }
 
 // ---- the closed form on the tensor cores (3-piece BF16 splits, FP32 accumulation): the three
@@ -782,10 +859,10 @@ __global__ void k_chunk_y(const float *__restrict__ Y, int N, int nao, int nch, 
     }
 }
 
-// H[e] = sum_c Hp[c][e] in FP64
-__global__ void k_sum_chunks(const float *__restrict__ Hp, long long nn, int nch, double *__restrict__ H)
+// H[e] = sum_c Hp[c][e] in FP64 over n elements of each chunk (chunks nn apart): the home rows
+__global__ void k_sum_chunks(const float *__restrict__ Hp, long long nn, long long n, int nch, double *__restrict__ H)
 {
-    for (long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; e < nn;
+    for (long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
          e += static_cast<long long>(gridDim.x) * blockDim.x)
     {
         double acc = 0.0;
@@ -804,8 +881,8 @@ struct HsSplitWork
 
 int pad64(long long n) { return static_cast<int>((n + 63) / 64 * 64); }
 
-void hs_closed_form_split(const GammaSetup &gs, const double *W, const double *const *D, int nd, double *const *H,
-                          HsSplitWork &wk, cudaStream_t st)
+void hs_closed_form_split(const GammaSetup &gs, const double *W, const double *D, int nd, double *H, HsSplitWork &wk,
+                          cudaStream_t st)
 {
     const int N = gs.N, nao = gs.nao;
     const long long nn = static_cast<long long>(nao) * nao, big = static_cast<long long>(N) * nn;
@@ -844,7 +921,7 @@ void hs_closed_form_split(const GammaSetup &gs, const double *W, const double *c
     for (int d = 0; d < nd; ++d)
     {
         // Y = U D: Y[(a, p)][s]
-        split_transpose_f64(D[d], nao, nao, nao, kpA, wk.Dsp.bufs(), st);
+        split_transpose_f64(D + d * nn, nao, nao, nao, kpA, wk.Dsp.bufs(), st);
         tc_gemm_split(wk.Ur.mat(static_cast<long long>(N) * nao, kpA, 0), wk.Dsp.mat(nao, kpA, 0), N * nao, nao, nao, 1,
                       wk.Yf.get(), nao, 0, false, wk.err.get(), st);
         k_chunk_y<<<grid_for(chunked), 256, 0, st>>>(wk.Yf.get(), N, nao, nch, wk.Yc.get());
@@ -854,7 +931,8 @@ void hs_closed_form_split(const GammaSetup &gs, const double *W, const double *c
         // H = sum over chunks of Yc[c] Zc[c]^T
         tc_gemm_split(wk.Ys.mat(nao, kc, static_cast<long long>(nao) * kc), wk.Zs.mat(nao, kc, static_cast<long long>(nao) * kc),
                       nao, nao, static_cast<int>(kc), nch, wk.Hp.get(), nao, nn, false, wk.err.get(), st);
-        k_sum_chunks<<<grid_for(nn), 256, 0, st>>>(wk.Hp.get(), nn, nch, H[d]);
+        const long long hn = static_cast<long long>(gs.naoc) * nao;
+        k_sum_chunks<<<grid_for(hn), 256, 0, st>>>(wk.Hp.get() + static_cast<long long>(gs.c0) * hn, nn, hn, nch, H + d * hn);
         GB_LAUNCH_CHECK();
     }
     int herr = 0;
@@ -877,7 +955,7 @@ struct SigmaClosedForm
         const long long nn = static_cast<long long>(gs.nao) * gs.nao;
         split = ds.gbopt.sigma_precision == LIBRPA_GB300_SIGMA_BF16X3 && (nn + 31) / 32 <= 65535;
     }
-    void run(const GammaSetup &gs, const double *W, const double *const *D, int nd, double *const *H, cudaStream_t st)
+    void run(const GammaSetup &gs, const double *W, const double *D, int nd, double *H, cudaStream_t st)
     {
         if (split)
             hs_closed_form_split(gs, W, D, nd, H, tc, st);
@@ -935,9 +1013,10 @@ void build_exx(Dataset &ds, const LibrpaOptions &opts)
     block_filter_host(vr, gs.Nc, gs.abf_off, opts.libri_exx_threshold_V);
     const std::vector<double> vs = to_supercell(vr, gs.Nc, gs);
     const long long nn = static_cast<long long>(nao) * nao;
-    DevBuf<double> dV(vs.size()), dD(nn), dH(nn);
+    const long long hn = static_cast<long long>(naoc) * nao;
+    DevBuf<double> dV(vs.size()), dD(nn), dH(hn);
     dV.upload(vs.data(), vs.size(), st);
-    std::vector<double> hs(nn);
+    std::vector<double> hs(hn);
     HsWork wk;  // FP64: v_exx is held to the reference's print precision
     ds.hx.assign(ns, {});
     ds.hx_r.assign(ns, {});
@@ -947,9 +1026,7 @@ void build_exx(Dataset &ds, const LibrpaOptions &opts)
         block_filter_host(dr, naoc, gs.ao_off, opts.libri_exx_threshold_D);
         const std::vector<double> dsup = to_supercell(dr, naoc, gs);
         dD.upload(dsup.data(), dsup.size(), st);
-        const double *Dp[1] = {dD.get()};
-        double *Hp[1] = {dH.get()};
-        hs_closed_form(gs, dV.get(), Dp, 1, Hp, wk, st);
+        hs_closed_form(gs, dV.get(), dD.get(), 1, dH.get(), wk, st);
         dH.download(hs.data(), hs.size(), st);
         GB_CUDA(cudaStreamSynchronize(st));
         // H(R_c)_KL: the supercell row block of the cell R = 0, column block of cell c
@@ -957,8 +1034,8 @@ void build_exx(Dataset &ds, const LibrpaOptions &opts)
         hr.resize(static_cast<size_t>(nc) * naoc * naoc);
         for (int c = 0; c < nc; ++c)
             for (int K = 0; K < naoc; ++K)
-                std::copy(hs.data() + (static_cast<size_t>(gs.c0) * naoc + K) * nao + static_cast<size_t>(c) * naoc,
-                          hs.data() + (static_cast<size_t>(gs.c0) * naoc + K) * nao + static_cast<size_t>(c + 1) * naoc,
+                std::copy(hs.data() + static_cast<size_t>(K) * nao + static_cast<size_t>(c) * naoc,
+                          hs.data() + static_cast<size_t>(K) * nao + static_cast<size_t>(c + 1) * naoc,
                           hr.data() + (static_cast<size_t>(c) * naoc + K) * naoc);
         ds.hx[s].assign(hr.begin() + static_cast<size_t>(gs.c0) * naoc * naoc,
                         hr.begin() + static_cast<size_t>(gs.c0 + 1) * naoc * naoc);
@@ -1107,7 +1184,8 @@ void build_g0w0_gamma(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
 
     // Sigma_c(i omega) = sum_tau [cos_t2f (S+ + S-)/2 + i sin_t2f (S+ - S-)/2] per spin, then the KS diagonal
     DevBuf<cuDoubleComplex> Sig(nn * nw), dpsi(static_cast<size_t>(nb) * nao), sks(static_cast<size_t>(nb) * nw);
-    DevBuf<double> sgn_s(2ull * nb), Gp(nn), Gm(nn), Sp(nn), Sm(nn), cw(nw), sw(nw);
+    DevBuf<double> sgn_s(2ull * nb), G(2 * nn), S2(2 * nn), cw(nw), sw(nw);
+    double *const Gp = G.get(), *const Gm = G.get() + nn, *const Sp = S2.get(), *const Sm = S2.get() + nn;
     SigmaClosedForm cf(ds, gs);
     // LibRI's set_Ws filter on every W(tau) (libri_g0w0_threshold_Wc; gw.cpp:459-470)
     auto d_aoo_f = to_dev(gs.ao_off, st);
@@ -1140,18 +1218,16 @@ void build_g0w0_gamma(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
                 sm[n] = std::exp(std::min(0.0, tau * e)) * wm;
             }
             sgn_s.upload(sp.data(), nb, st);
-            k_gamma_dm<<<(nao * nao + 255) / 256, 256, 0, st>>>(dpsi.get(), sgn_s.get(), nb, nao, 1.0, Gp.get());
+            k_gamma_dm<<<(nao * nao + 255) / 256, 256, 0, st>>>(dpsi.get(), sgn_s.get(), nb, nao, 1.0, Gp);
             GB_LAUNCH_CHECK();
             GB_CUDA(cudaStreamSynchronize(st));
             sgn_s.upload(sm.data(), nb, st);
-            k_gamma_dm<<<(nao * nao + 255) / 256, 256, 0, st>>>(dpsi.get(), sgn_s.get(), nb, nao, -1.0, Gm.get());
+            k_gamma_dm<<<(nao * nao + 255) / 256, 256, 0, st>>>(dpsi.get(), sgn_s.get(), nb, nao, -1.0, Gm);
             GB_LAUNCH_CHECK();
             // LibRI's set_Gs filter (libri_g0w0_threshold_G; gw.cpp:546-616)
-            block_filter_dev(Gp.get(), 0, 1, 0, 1, nao, d_aoo_f.get(), gs.n_at, opts.libri_g0w0_threshold_G, st);
-            block_filter_dev(Gm.get(), 0, 1, 0, 1, nao, d_aoo_f.get(), gs.n_at, opts.libri_g0w0_threshold_G, st);
-            const double *Dp[2] = {Gp.get(), Gm.get()};
-            double *Hp[2] = {Sp.get(), Sm.get()};
-            cf.run(gs, Wt.get() + it * NN, Dp, 2, Hp, st);
+            block_filter_dev(Gp, 0, 1, 0, 1, nao, d_aoo_f.get(), gs.n_at, opts.libri_g0w0_threshold_G, st);
+            block_filter_dev(Gm, 0, 1, 0, 1, nao, d_aoo_f.get(), gs.n_at, opts.libri_g0w0_threshold_G, st);
+            cf.run(gs, Wt.get() + it * NN, G.get(), 2, S2.get(), st);
             std::vector<double> c(nw), sn(nw);
             for (int w = 0; w < nw; ++w)
             {
@@ -1160,7 +1236,7 @@ void build_g0w0_gamma(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
             }
             cw.upload(c.data(), nw, st);
             sw.upload(sn.data(), nw, st);
-            k_sigma_accumulate<<<grid_for(nn * nw), 256, 0, st>>>(Sp.get(), Sm.get(), static_cast<int>(nn), cw.get(),
+            k_sigma_accumulate<<<grid_for(nn * nw), 256, 0, st>>>(Sp, Sm, static_cast<int>(nn), cw.get(),
                                                                    sw.get(), nw, Sig.get());
             GB_LAUNCH_CHECK();
             GB_CUDA(cudaStreamSynchronize(st));  // the host weight vectors are reused
@@ -1514,8 +1590,9 @@ void build_g0w0_kgrid(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
     auto d_gcos = to_dev(pt.gcos, st);
     auto d_gsin = to_dev(pt.gsin, st);
     auto d_cdiff = to_dev(gs.cdiff, st);
-    DevBuf<double> d_s(2ull * nk * nb), d_G(2ull * nc * nnc), Ws(static_cast<size_t>(gs.N) * gs.N), Gps(ns2), Gms(ns2),
-        Sp(ns2), Sm(ns2), cw(nw), sw(nw);
+    const long long hn = nnc * nc;  // Sigma of the home rows: [n_ao][supercell NAO]
+    DevBuf<double> d_s(2ull * nk * nb), d_G(2ull * nc * nnc), Ws(static_cast<size_t>(gs.N) * gs.N), Gs(2 * ns2), S2(2 * hn),
+        cw(nw), sw(nw);
     DevBuf<cuDoubleComplex> d_A(2ull * nk * nnc), Sig(static_cast<size_t>(nw) * nc * nnc);
     SigmaClosedForm cf(ds, gs);
     ds.sigc_ks.assign(ns, {});
@@ -1532,14 +1609,12 @@ void build_g0w0_kgrid(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
             launch_phase_sum(d_A.get(), d_gcos.get(), d_gsin.get(), nk, nc, nao, d_G.get(), st);
             // LibRI's set_Gs filter on G(R, +-tau) (libri_g0w0_threshold_G; gw.cpp:546-616)
             block_filter_dev(d_G.get(), nnc, 2 * nc, 0, 1, nao, d_aoo_f.get(), n_at, opts.libri_g0w0_threshold_G, st);
-            k_to_super<<<grid_for(ns2), 256, 0, st>>>(d_G.get(), nnc, nao, nc, d_cdiff.get(), Gps.get());
-            k_to_super<<<grid_for(ns2), 256, 0, st>>>(d_G.get() + nc * nnc, nnc, nao, nc, d_cdiff.get(), Gms.get());
+            k_to_super<<<grid_for(ns2), 256, 0, st>>>(d_G.get(), nnc, nao, nc, d_cdiff.get(), Gs.get());
+            k_to_super<<<grid_for(ns2), 256, 0, st>>>(d_G.get() + nc * nnc, nnc, nao, nc, d_cdiff.get(), Gs.get() + ns2);
             k_to_super<<<grid_for(static_cast<long long>(gs.N) * gs.N), 256, 0, st>>>(
                 Wt.get() + static_cast<long long>(it) * NN, nw * NN, Nc, nc, d_cdiff.get(), Ws.get());
             GB_LAUNCH_CHECK();
-            const double *Dp[2] = {Gps.get(), Gms.get()};
-            double *Hp[2] = {Sp.get(), Sm.get()};
-            cf.run(gs, Ws.get(), Dp, 2, Hp, st);
+            cf.run(gs, Ws.get(), Gs.get(), 2, S2.get(), st);
             std::vector<double> c(nw), sn(nw);
             for (int w = 0; w < nw; ++w)
             {
@@ -1548,8 +1623,8 @@ void build_g0w0_kgrid(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
             }
             cw.upload(c.data(), nw, st);
             sw.upload(sn.data(), nw, st);
-            k_sigma_rows<<<grid_for(nnc * nc * nw), 256, 0, st>>>(Sp.get(), Sm.get(), gs.c0, nc, nao, cw.get(), sw.get(),
-                                                                  nw, Sig.get());
+            k_sigma_rows<<<grid_for(nnc * nc * nw), 256, 0, st>>>(S2.get(), S2.get() + hn, nc, nao, cw.get(), sw.get(), nw,
+                                                                  Sig.get());
             GB_LAUNCH_CHECK();
             GB_CUDA(cudaStreamSynchronize(st));  // the host weight vectors are reused
         }
