@@ -9,11 +9,10 @@
 //        E[(cJ,mu)][j, K'] = sum_i Ga[cJ]_{ij} X_b^I[mu i][shift_cJ(K')]
 //     where K' runs over the supercell orbitals (cell R', atom L, orbital l) of C^J's own
 //     frame and shift_cJ maps R' -> R' + R_cJ (the T1 term with R_L = R' + R_J).
-//     Eight producer warps form E in FP32 on the CUDA cores (packed FP32x2 FMAs, 4 columns a
-//     thread), split it into BF16 pieces and
-//     write the 128 x 64 A tile of each pipeline stage into swizzled shared memory; one lane
-//     streams the matching C^J tile (64 K-elements per row, pre-arranged in HBM) with TMA and
-//     one lane issues the tcgen05.mma terms.  K order: pass, 8-column chunk, group of 8 j.
+//     Eight producer warps form E in FP32 on the CUDA cores (packed FP32x2 FMAs, a row and 8 columns
+//     a thread), split it into BF16 pieces and write them to TMEM, where the MMAs read A; one lane
+//     streams the matching C^J tiles (64 K-elements per row, pre-arranged in HBM) with TMA and issues
+//     the tcgen05.mma terms.  K order: 8-column chunk, group of 8 j.
 //  3. T2 (small, CUDA cores): D += sum_{i,j} X_b^I[mu i; (cJ,J) j] X_a^J[nu j; (-cJ,I) i].
 // Every wait is bounded (tc_common.cuh) and failures surface through a device error flag.
 #include <algorithm>
@@ -36,30 +35,23 @@ using namespace tc;
 
 constexpr int NS = 3;            // BF16 pieces per operand (hi, mid, lo): 6 MMA terms
 constexpr int T1_BM = 128;       // rows (cJ, mu) per CTA
-constexpr int CW = 8;            // supercell columns per chunk
+constexpr int CW = 8;            // supercell columns per chunk: two groups of 4 columns of one cell each
 constexpr int JG = 8;            // j per pipeline stage (JG * CW = 64 = K per stage)
-constexpr int T1_STAGES = 2;     // A (E tile) ring: producers fill one while the MMAs read the other
 constexpr int T1_MAXB = 8;       // C^J (B tile) ring: up to 8 stages of TMA look-ahead
 constexpr int T1_NMAX = 128;     // max N tile (ABFs of one atom, padded to 16)
-// Two producer layouts.  Wide (P2 = false): warps 0-7 build E, 2 threads per row with 4
-// columns each; 12 warps, up to 168 registers a thread.  Narrow (P2 = true, the streamed
-// 4-column-aligned case): warps 0-15 build E, 4 threads per row with 2 columns each, so twice
-// the warps hide the X gather latency; 20 warps, up to 102 registers a thread.  In both, the
-// 4 warps after the producers drain the accumulators, and lane 0 of the first of them also
-// issues the C^J TMA copies and the MMAs.
-template <bool P2>
-struct T1Layout
-{
-    static constexpr int producers = P2 ? 512 : 256;
-    static constexpr int drain_warp0 = producers / 32;
-    static constexpr int threads = producers + 128;
-};
-constexpr int A_TILE = T1_BM * 64 * 2;       // bytes per A piece
-constexpr int T1_MAXA = 32;                  // max NAOs per atom (G buffer row stride)
+constexpr int T1_SET = 128;      // producer threads per warpgroup: one row each
+constexpr int T1_PRODUCERS = 2 * T1_SET;           // two warpgroups, on alternate chunks
+constexpr int T1_DRAIN = T1_PRODUCERS / 32;        // first of the four drain warps
+constexpr int T1_ISSUE = T1_DRAIN + 4;             // one lane issues the MMAs and the C^J copies
+constexpr int T1_THREADS = T1_PRODUCERS + 256;     // four warpgroups (the last one has three idle warps)
+constexpr int T1_TMEM = 512;                       // TMEM columns: accumulators from 0, the A tiles at the end
+constexpr int T1_ACOLS = NS * 32;                  // columns of one A tile: 3 pieces x 64 BF16 of K
+constexpr int T1_ABASE = T1_TMEM - 2 * T1_ACOLS;   // one A tile per producer warpgroup
+constexpr int T1_MAXA = 32;                        // max NAOs per atom
+constexpr int T1_CELLS = 32;                       // cells of a row group's shift table in shared memory
 constexpr int T1_SMEM_MAX = 227 * 1024;
-// Shared memory: T1_STAGES x NS A pieces | nbs x NS B pieces of b_tile bytes | G blocks | barriers.
-// b_tile = NT_max * 128 rounded up to 1024; G blocks hold, per pass and cell, rap(RA) rows i
-// of gj FP32 entries j.
+// Shared memory: nbs x NS B pieces of b_tile bytes | X ring | G blocks | barriers.  b_tile = NT_max * 128
+// rounded up to 1024; a G block holds, per 8 j, the 2 n_ao(I) rows q = (pass, i).
 
 // A row group: the n_abf(I) rows mu of one chi0 block (pair (I, J), cell cJ).
 struct T1Group
@@ -96,21 +88,21 @@ struct T1Args
 {
     Geom g;
     Pairs pr;
-    const float *X;          // [2][rows_c][n_sup]: sign 0 = X(+), sign 1 = X(-)
-    long long xsign;         // rows_c * n_sup
+    const float4 *Xt;        // X in 4-column groups (k_x_layout)
+    const long long *xoff;   // [n_at] first float4 of each atom there
     const double *G;         // [2][n_c][n_ao][n_ao]
     const int *cadd;         // [n_c*n_c] cadd[a*n_c+b] = cell of R_a + R_b
     const T1Work *work;
     const T1Group *groups;
     const int *spec;           // [n_at] species of each atom
     const int *spec_idx;       // [n_at] index of the atom inside its species
-    const int *aJpad;          // NAOs of each atom rounded up to JG
-    int nkc;                   // number of CW-wide chunks of the supercell axis
+    int n4;                    // 4-column groups of one cell (NAOs rounded up to 4)
+    int ng4;                   // of the supercell: n_c * n4
     int b_tile;                // bytes per B piece (1024-aligned)
     int nbs;                   // stages of the B ring (2..T1_MAXB)
-    int gj;                    // j entries per i row of the G blocks (largest aJpad)
+    int gq;                    // rows q of the G blocks' parts of 8 j
+    int gslot;                 // floats per G block
     int maxcj;                 // most row groups a 128-row tile can touch
-    int vec4;                  // n_ao % 4 == 0: 4-column X gathers are one aligned float4
     double *out;               // chi0R
     int *err;
 };
@@ -120,78 +112,240 @@ __device__ __forceinline__ void named_bar_sync(int id, int n)
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
-__host__ __device__ constexpr int rap(int ra) { return (ra + 1) & ~1; }
-
 __device__ __forceinline__ uint32_t bf2_bits(__nv_bfloat162 h)
 {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
 // Three-piece BF16 split of a pair of FP32 values (hi, mid, lo), each piece packed as bf16x2
-// (element 0 in the low half): hi = rn(e), mid = rn(e - hi), lo = rn(e - hi - mid).
+// (element 0 in the low half).  Each piece takes the top 8 bits of what is left of the 24, so the three
+// together are the value exactly.  By masks and byte permutes: a float to BF16 conversion instruction
+// costs several times theirs.
 __device__ __forceinline__ void split3_pair(float2 e, uint32_t &h, uint32_t &m, uint32_t &l)
 {
+    constexpr uint32_t top = 0xffff0000u;
     const float2 neg1 = make_float2(-1.0f, -1.0f);
-    const __nv_bfloat162 hh = __floats2bfloat162_rn(e.x, e.y);
-    const float2 r1 = __ffma2_rn(__bfloat1622float2(hh), neg1, e);
-    const __nv_bfloat162 mm = __floats2bfloat162_rn(r1.x, r1.y);
-    const float2 r2 = __ffma2_rn(__bfloat1622float2(mm), neg1, r1);
-    h = bf2_bits(hh);
-    m = bf2_bits(mm);
-    l = bf2_bits(__floats2bfloat162_rn(r2.x, r2.y));
+    uint32_t x = __float_as_uint(e.x), y = __float_as_uint(e.y);
+    h = __byte_perm(x, y, 0x7632);
+    const float2 r1 = __ffma2_rn(make_float2(__uint_as_float(x & top), __uint_as_float(y & top)), neg1, e);
+    x = __float_as_uint(r1.x);
+    y = __float_as_uint(r1.y);
+    m = __byte_perm(x, y, 0x7632);
+    const float2 r2 = __ffma2_rn(make_float2(__uint_as_float(x & top), __uint_as_float(y & top)), neg1, r1);
+    l = __byte_perm(__float_as_uint(r2.x), __float_as_uint(r2.y), 0x7632);
 }
 
-// RA: register blocking over the NAOs i of atom I (13, 16 or 32: at least the largest NAO
-// count); NTC: accumulator columns held by the drain warps (64 or 128).
+// A = E in TMEM: D(tmem) (+)= A(tmem) * B(smem desc)^T, BF16 inputs, FP32 accumulate.  Row r of A is
+// TMEM lane r, each 32-bit column two consecutive K elements.
+__device__ __forceinline__ void mma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate)
+{
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(
+            d_tmem),
+        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// 16 consecutive 32-bit columns of the warp's 32 TMEM lanes
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// X reaches a producer through its own slots of a shared-memory ring, filled by 16-byte asynchronous
+// copies T1_XR - 1 blocks of T1_XD rows q ahead: a register ring of that depth does not fit beside E.
+constexpr int T1_XD = 4;
+constexpr int T1_XR = 3;
+// rows q = (pass, i) of X kept for an atom: whole blocks, the last ones zero
+__host__ __device__ constexpr int t1_rows(int nao) { return (2 * nao + T1_XD - 1) / T1_XD * T1_XD; }
+constexpr int T1_XBYTES = T1_XR * T1_XD * 2 * T1_PRODUCERS * 16;
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool live)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// The place in X a producer's copies have reached: chunk kc, unit un of its j, row q of that unit, and
+// the chunk's two 4-column groups (offset of their row 0 from the thread's row, in float4; live: inside
+// the supercell and the tile's rows, else zero-filled).
+struct T1Cursor
+{
+    int kc, un, q;
+    uint32_t off[2];
+    bool live[2];
+};
+
+__device__ __forceinline__ float4 lds128(uint32_t addr)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+    return v;
+}
+
+// One row q: E[j][col] += G[q][j] X[q][col], columns in pairs
+template <int NJ>
+__device__ __forceinline__ void t1_row(uint32_t xs, uint32_t ga, uint32_t gb, float2 (&e)[NJ][CW / 2])
+{
+    const float4 x0 = lds128(xs), x1 = lds128(xs + T1_PRODUCERS * 16);
+    const float2 xp[CW / 2] = {make_float2(x0.x, x0.y), make_float2(x0.z, x0.w), make_float2(x1.x, x1.y),
+                               make_float2(x1.z, x1.w)};
+#pragma unroll
+    for (int jh = 0; jh < (NJ + 3) / 4; ++jh)
+    {
+        const float4 gg = lds128(jh < 2 ? ga + jh * 16 : gb + (jh - 2) * 16);
+        const float gv[4] = {gg.x, gg.y, gg.z, gg.w};
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (4 * jh + t < NJ)
+            {
+                const float2 g2 = make_float2(gv[t], gv[t]);
+#pragma unroll
+                for (int c = 0; c < CW / 2; ++c) e[4 * jh + t][c] = __ffma2_rn(g2, xp[c], e[4 * jh + t][c]);
+            }
+    }
+}
+
+// One unit of a producer thread's work: its row r, one chunk of 8 columns and NJ <= JT consecutive j,
+//   E[j][col] = sum_q G[q][j] X[q][col],   q = (pass, i),
+// then its 3-piece BF16 split, written to the warpgroup's A tile in TMEM half a stage (4 j) at a time.
+//
+// Bounds: 128 FP32 FMAs per clock per SM (the rows loop alone reaches 92), next to it the shared-memory
+// path: a G value loaded serves the thread's 8 columns, an X value its j.  The two warpgroups work on
+// alternate chunks, so that the split and the hand-over of one run under the FMAs of the other.
+// Measured (13 NAO / 40 ABF atoms, per tau): 128 atoms at Gamma 21.2 -> 13.6 ms, 8 -> 12 mixed-species
+// atoms a tile (5/20, 13/60, 26/110; 48 atoms) 20.0 -> 4.0 ms, against two threads a row that wrote E to
+// shared memory with one drain warp issuing everything.  What is left: the producers' two warps per
+// scheduler, 48 of 128 FMAs per clock over the whole kernel.
+template <int NJ, typename Fetch>
+__device__ __forceinline__ bool t1_unit(uint32_t xring, int &slot, const Fetch &fetch, uint32_t gs,
+                                        int gq, int nq, int nhalf, uint32_t atile, uint64_t *full, uint64_t *empty, uint32_t &use,
+                                        int lane, int *err)
+{
+    constexpr uint32_t GQ = JG * 4;  // bytes of a row q of 8 G values
+    float2 e[NJ][CW / 2];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int c = 0; c < CW / 2; ++c) e[j][c] = make_float2(0.f, 0.f);
+    uint32_t ga = gs, gb = gs + gq * GQ;  // j 0..7 and 8..15
+    for (int left = nq; left > 0; left -= T1_XD)
+    {
+        fetch(slot);  // refills the slot read in the previous round
+        cp_async_wait<T1_XR - 1>();
+        uint32_t xs = xring + slot * (T1_XD * 2 * T1_PRODUCERS * 16);
+        slot = slot + 1 == T1_XR ? 0 : slot + 1;
+        // two rows at a time (nq is even): unrolled further, the rows' loads crowd E out of the registers
+#pragma unroll 1
+        for (int r = min(left, T1_XD); r > 0; r -= 2)
+        {
+            t1_row<NJ>(xs, ga, gb, e);
+            t1_row<NJ>(xs + 2 * T1_PRODUCERS * 16, ga + GQ, gb + GQ, e);
+            xs += 4 * T1_PRODUCERS * 16;
+            ga += 2 * GQ;
+            gb += 2 * GQ;
+        }
+    }
+    // half stages of 4 j x 8 columns (K = 32): the split of one runs under the MMAs of the one before
+#pragma unroll
+    for (int hs = 0; hs < (NJ + 3) / 4; ++hs)
+    {
+        if (hs >= nhalf) break;  // the half stages the issue warp counts
+        const int h = hs & 1;
+        uint32_t wh[16], wm[16], wl[16];  // 16 TMEM columns of each piece
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int c = 0; c < CW / 2; ++c)
+            {
+                const int j = hs * 4 + t;
+                if (j < NJ)
+                    split3_pair(e[j < NJ ? j : 0][c], wh[t * 4 + c], wm[t * 4 + c], wl[t * 4 + c]);
+                else
+                    wh[t * 4 + c] = wm[t * 4 + c] = wl[t * 4 + c] = 0u;
+            }
+        // half h of the A tile is free once the MMAs of its previous use are done
+        if (!__all_sync(0xffffffffu, mbar_wait_nap<0>(empty + h, (use >> h) & 1)))
+        {
+            if (lane == 0) atomicExch(err, 201);
+            return false;
+        }
+        use ^= 1u << h;
+        tc_fence_after();
+        tmem_st16(atile + h * 16, wh);
+        tmem_st16(atile + 32 + h * 16, wm);
+        tmem_st16(atile + 64 + h * 16, wl);
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full + h);
+    }
+    return true;
+}
+
+// NTC: accumulator columns held by the drain warps (48, 64 or 128: at least the largest N tile).
 //
 // Both LibRI passes share the B operand C^J, so one A tile carries E(+) + E(-) (pass 0:
-// G(+) with X(-), pass 1: G(-) with X(+)) and each K step is contracted once.  With NTC = 64
+// G(+) with X(-), pass 1: G(-) with X(+)) and each K step is contracted once.  Up to NTC = 64
 // the three C^J pieces sit on top of each other along N and each K16 step is three MMAs,
 // hi x [Ch;Cm;Cl] (N = 3 NT), mid x [Ch;Cm] (N = 2 NT) and lo x Ch (N = NT), landing in three
 // accumulator blocks of orders 1, 2^-8 and 2^-16; with NTC = 128 the six products are issued
 // one by one into a hi*hi block and a cross-term block.
-template <int RA, int NTC, bool SV, bool P2>
-__global__ void __launch_bounds__(T1Layout<P2>::threads, 1) k_t1_tc(const __grid_constant__ T1Args a,
-                                                                   const __grid_constant__ T1Maps maps)
+//
+// The A tile goes from the producers' registers to TMEM and is read there by the MMAs: neither the
+// 48 KB a stage of E nor its re-reads by the MMAs pass through shared memory, whose bandwidth bounds
+// the producers.  TMEM: 512 columns = accumulators (two buffers where they fit, else one) + two A tiles.
+// The MMAs and the C^J copies are issued by a warp of their own: issued from a drain warp they cost that
+// warp's loop 4900 clocks a stage, which bounded the whole contraction.
+//
+// Registers: a producer holds up to JT j x 8 columns of E, a drain warp NTC accumulator columns; the
+// warpgroups trade registers (setmaxnreg) so that 2 PREG + DREG + CREG = 4 x 128, the launch's share.
+template <int NTC>
+__global__ void __launch_bounds__(T1_THREADS, 1) k_t1_tc(const __grid_constant__ T1Args a,
+                                                         const __grid_constant__ T1Maps maps)
 {
-    constexpr int PRODUCERS = T1Layout<P2>::producers;
-    constexpr int DRAIN_WARP0 = T1Layout<P2>::drain_warp0;
-    constexpr bool STACKN = NTC == 64;
+    constexpr bool STACKN = NTC <= 64;
     constexpr int NBLK = STACKN ? 3 : 2;           // accumulator blocks per buffer
-    constexpr uint32_t TMEM_COLS = 512;
-    static_assert(2 * NBLK * NTC <= static_cast<int>(TMEM_COLS), "TMEM budget");
-    constexpr int RP = rap(RA);
-    constexpr bool BOTHX = RA <= 13;  // keep both passes' X values of a chunk in registers
-    // SV: 4-column X gathers are aligned (n_ao % 4 == 0), so the producers stream X through a
-    // register ring, one chunk (both stages, up to 16 j) per pass; otherwise the gathers go one
-    // column at a time below
-    constexpr bool STREAM = SV && RA <= 16 && JG == 8;
-    static_assert(!P2 || STREAM, "the narrow producer layout streams 4-column-aligned X");
+    constexpr int JT = STACKN ? 16 : 8;            // most j per unit of the producers
+    constexpr int PREG = STACKN ? 192 : 160, DREG = NTC == 48 ? 96 : NTC == 64 ? 104 : 168, CREG = NTC == 48 ? 32 : 24;
+    static_assert(2 * PREG + DREG + CREG == 4 * 128, "register split of the launch's 128 a thread");
+    static_assert(NBLK * NTC <= T1_ABASE, "TMEM budget");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int stage_bytes = NS * A_TILE;      // A ring stage
+    unsigned char *bring = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int bstage_bytes = NS * a.b_tile;   // B ring stage
     const int nbs = a.nbs;
-    const int gst = a.gj;                     // j entries per i row of a G block
-    const int g_floats = 2 * a.maxcj * RP * gst;
-    unsigned char *bring = smem + T1_STAGES * stage_bytes;
-    float *gsm = reinterpret_cast<float *>(bring + nbs * bstage_bytes);
-    uint64_t *full = reinterpret_cast<uint64_t *>(gsm + g_floats);  // A ring: producers filled
-    uint64_t *empty = full + T1_STAGES;                              // A ring: MMAs done
-    uint64_t *bfull = empty + T1_STAGES;                             // B ring: TMA landed
-    uint64_t *bempty = bfull + T1_MAXB;                              // B ring: MMAs done
+    const int gq = a.gq;                      // rows q of a G block's part of 8 j
+    unsigned char *xring = bring + nbs * bstage_bytes;
+    float *gsm = reinterpret_cast<float *>(xring + T1_XBYTES);
+    uint64_t *full = reinterpret_cast<uint64_t *>(gsm + a.maxcj * (a.gslot + T1_CELLS));  // [set][half] A tile: written
+    uint64_t *empty = full + 4;                                              // A tile: MMAs done
+    uint64_t *bfull = empty + 4;                                             // B ring: TMA landed
+    uint64_t *bempty = bfull + T1_MAXB;                                      // B ring: MMAs done
     uint64_t *accf = bempty + T1_MAXB;
     uint64_t *acce = accf + 2;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acce + 2);
+    uint64_t *fin = acce + 2;                                                // every issued MMA done
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fin + 1);
+    volatile int *drain_stop = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const Geom &g = a.g;
     const T1Work w = a.work[blockIdx.x];
     const int J = w.J;
     const int aJ = g.nao[J], bJ = g.nabf[J];
-    const int njg = a.aJpad[J] / JG;
+    const int njg = (aJ + JG - 1) / JG;
     const int NT = (bJ + 15) / 16 * 16;
+    const int nab = 2 * NBLK * NT <= T1_ABASE ? 2 : 1;  // accumulator buffers
     const int nc = g.n_c, nao = g.n_ao;
-    const long long nsup = g.n_sup;
     // row r of the tile -> (row group, mu); false beyond the tile's valid rows
     auto row_of = [&](int r, int &grp, int &mu) -> bool {
         if (r >= w.nrows) return false;
@@ -215,573 +369,335 @@ __global__ void __launch_bounds__(T1Layout<P2>::threads, 1) k_t1_tc(const __grid
 
     if (threadIdx.x == 0)
     {
-        for (int s = 0; s < T1_STAGES; ++s)
+        for (int s = 0; s < 4; ++s)
         {
-            mbar_init(&full[s], PRODUCERS / 32);  // one arrival per producer warp
+            mbar_init(&full[s], T1_SET / 32);  // one arrival per producer warp
             mbar_init(&empty[s], 1);
         }
+        for (int s = 0; s < 2; ++s)
+        {
+            mbar_init(&accf[s], 1);
+            mbar_init(&acce[s], 4);            // one arrival per drain warp
+        }
+        mbar_init(fin, 1);
+        *drain_stop = 0;
         for (int s = 0; s < nbs; ++s)
         {
             mbar_init(&bfull[s], 1);
             mbar_init(&bempty[s], 1);
         }
-        for (int i = 0; i < 2; ++i)
-        {
-            mbar_init(&accf[i], 1);
-            mbar_init(&acce[i], 4);               // one arrival per drain warp
-        }
         fence_barrier_init();
     }
-    if (warp == 0) tmem_alloc(tmem_slot, TMEM_COLS);
+    if (warp == 0) tmem_alloc(tmem_slot, T1_TMEM);
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    if (threadIdx.x < PRODUCERS)
+    if (threadIdx.x < T1_PRODUCERS)
     {
         // ---------------- producers: E tiles
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PREG));
         const int t = threadIdx.x;
-        const int r = P2 ? t >> 2 : t >> 1;  // row in tile
-        const int cq = P2 ? t & 3 : t & 1;   // 2- (narrow) or 4-column (wide) group inside the 8-column chunk
-        int grp = 0, mu = 0;
-        const bool valid = row_of(r, grp, mu);
-        const int slot = valid ? grp - w.g0 : 0;
-        const int I = a.pr.I[a.groups[valid ? grp : w.g0].pair];
-        const int cJ = valid ? a.groups[grp].cell : 0;
-        const int aI = g.nao[I];
-        const long long xrow = g.rowc_off[I] + static_cast<long long>(mu) * aI;
-        // G blocks of both passes for the tile's row groups, [pass][slot][i][j] in FP32
-        const int per_pass = w.nslot * RP * gst;
-        for (int e = t; e < 2 * per_pass; e += PRODUCERS)
+        const int set = t / T1_SET;  // chunks kc0 + set, kc0 + set + 2, ...
+        int grp = w.g0, mu = 0;
+        const bool valid = row_of(t % T1_SET, grp, mu);
+        const int I = a.pr.I[a.groups[grp].pair];
+        const int cJ = a.groups[grp].cell;
+        const int aI = g.nao[I], bI = g.nabf[I];
+        const float4 *xrow = a.Xt + a.xoff[I] + mu;
+        // G blocks of the tile's row groups, [slot][j / 8][q = (pass, i)][j % 8] in FP32 (zero rows past
+        // 2 a_I, zero past a_J)
+        const int nq = 2 * w.ra;
+        for (int s = 0; s < w.nslot; ++s)
         {
-            const int pass = e / per_pass, rem = e % per_pass;
-            const int sl = rem / (RP * gst), ij = rem % (RP * gst);
-            const int i = ij / gst, j = ij % gst;
-            const T1Group gr = a.groups[w.g0 + sl];
-            const int Ig = a.pr.I[gr.pair];
-            float v = 0.0f;
-            if (i < g.nao[Ig] && j < aJ)
-                v = static_cast<float>(a.G[((static_cast<size_t>(pass) * nc + gr.cell) * nao + g.ao_off[Ig] + i) * nao +
-                                           g.ao_off[J] + j]);
-            gsm[(static_cast<size_t>(pass) * a.maxcj + sl) * RP * gst + ij] = v;
+            const T1Group gr = a.groups[w.g0 + s];
+            const int Ig = a.pr.I[gr.pair], ag = g.nao[Ig];
+            for (int e = t; e < njg * nq * JG; e += T1_PRODUCERS)
+            {
+                const int jg = e / (nq * JG), q = e / JG % nq, j = jg * JG + e % JG;
+                const int pass = q >= ag, i = pass ? q - ag : q;
+                float v = 0.0f;
+                if (q < 2 * ag && j < aJ)
+                    v = static_cast<float>(a.G[((static_cast<size_t>(pass) * nc + gr.cell) * nao + g.ao_off[Ig] + i) * nao +
+                                               g.ao_off[J] + j]);
+                gsm[s * a.gslot + (jg * gq + q) * JG + e % JG] = v;
+            }
         }
-        named_bar_sync(1, PRODUCERS);
-        const float4 *gp[2];
+        // cells of the shifted columns of each row group: R' + R_cJ (kept in shared memory for up to
+        // T1_CELLS cells, read once per chunk)
+        int *ctab = reinterpret_cast<int *>(gsm + a.maxcj * a.gslot);
+        if (nc <= T1_CELLS)
+            for (int e = t; e < w.nslot * nc; e += T1_PRODUCERS)
+                ctab[e / nc * T1_CELLS + e % nc] = a.cadd[(e % nc) * nc + a.groups[w.g0 + e / nc].cell];
+        const int *crow = nc <= T1_CELLS ? ctab + (grp - w.g0) * T1_CELLS : nullptr;
+        named_bar_sync(1, T1_PRODUCERS);
+        const uint32_t gs = smem_u32(gsm + (grp - w.g0) * a.gslot);
+        // units of j: all of an atom of 9 to 14 NAOs at once, 8 at a time otherwise (E of a thread's row
+        // and chunk is 14 x 8 registers at most)
+        const bool wide = JT == 16 && aJ > 8 && aJ <= 14;
+        const int nunit = wide ? 1 : njg;
+        T1Cursor cur;
+        auto point_at = [&](int kc) {
+            cur.kc = kc;
+            cur.un = 0;
+            cur.q = 0;
 #pragma unroll
-        for (int pass = 0; pass < 2; ++pass)
-            gp[pass] = reinterpret_cast<const float4 *>(gsm) + (static_cast<size_t>(pass) * a.maxcj + slot) * RP * gst / 4;
-        const float *Xp[2] = {a.X + a.xsign, a.X};  // pass 0 contracts G(+) with X(-), pass 1 G(-) with X(+)
-        // X_b^I[mu i][shift_cJ(col)] for the thread's 4 columns of chunk kc (np passes from pass p0)
-        // The tile's i range: row groups of one NAO count share tiles, so on a tile of small
-        // atoms the loops over i stop at its own count (a CTA-uniform branch), not at RA.
-        const int ira = w.ra;
-        auto load_x = [&](int kc, int p0, int np, float4 (&x0)[RA], float4 (&x1)[BOTHX ? RA : 1]) {
-            const long long col0 = static_cast<long long>(kc) * CW + cq * 4;
-            if (a.vec4)
+            for (int h = 0; h < 2; ++h)
             {
-                long long src = -1;
-                if (col0 < nsup && valid)
+                const int g4 = 2 * kc + h;
+                cur.off[h] = 0;
+                cur.live[h] = valid && kc < kc1 && g4 < a.ng4;
+                if (cur.live[h])
                 {
-                    const int cp = static_cast<int>(col0 / nao), ao = static_cast<int>(col0 % nao);
-                    src = static_cast<long long>(a.cadd[cp * nc + cJ]) * nao + ao;
-                }
-                const float *b0 = Xp[p0] + xrow * nsup + src;
-#pragma unroll
-                for (int i = 0; i < RA; ++i)
-                    if (i < ira) x0[i] = (i < aI && src >= 0) ? __ldg(reinterpret_cast<const float4 *>(b0 + i * nsup))
-                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
-                if constexpr (BOTHX)
-                    if (np == 2)
-                    {
-                        const float *b1 = Xp[p0 + 1] + xrow * nsup + src;
-#pragma unroll
-                        for (int i = 0; i < RA; ++i)
-                            if (i < ira) x1[i] = (i < aI && src >= 0) ? __ldg(reinterpret_cast<const float4 *>(b1 + i * nsup))
-                                                         : make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
-            }
-            else
-            {
-                long long src[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                {
-                    const long long col = col0 + q;
-                    src[q] = -1;
-                    if (col < nsup && valid)
-                    {
-                        const int cp = static_cast<int>(col / nao), ao = static_cast<int>(col % nao);
-                        src[q] = static_cast<long long>(a.cadd[cp * nc + cJ]) * nao + ao;
-                    }
-                }
-                auto gather = [&](const float *Xb, float4(&x)[RA]) {
-#pragma unroll
-                    for (int i = 0; i < RA; ++i)
-                    {
-                        if (i >= ira) continue;
-                        const float *xr = Xb + (xrow + i) * nsup;
-                        const bool ri = i < aI;
-                        x[i] = make_float4(ri && src[0] >= 0 ? xr[src[0]] : 0.f, ri && src[1] >= 0 ? xr[src[1]] : 0.f,
-                                           ri && src[2] >= 0 ? xr[src[2]] : 0.f, ri && src[3] >= 0 ? xr[src[3]] : 0.f);
-                    }
-                };
-                gather(Xp[p0], x0);
-                if constexpr (BOTHX)
-                    if (np == 2) gather(Xp[p0 + 1], x1);
-            }
-        };
-        // E[j][col pair] += sum_i g_ij x_i for JH consecutive j from j0
-        constexpr int JH = JG / 2;
-        auto contract = [&](const float4 *gb, int j0, const float4 (&x)[RA], float2 (&e)[JH][2]) {
-#pragma unroll
-            for (int i = 0; i < RA; ++i)
-            {
-                if (i >= ira) continue;
-                // one 16-byte load gives g_ij for the JH = 4 values of j; each is paired {g, g}
-                // in registers as the broadcast operand of the packed FMAs
-                static_assert(JH == 4, "one float4 of G per (i, half stage)");
-                const float4 gg = gb[(i * gst + j0) / 4];
-                const float2 xa = make_float2(x[i].x, x[i].y), xb = make_float2(x[i].z, x[i].w);
-                const float gv[4] = {gg.x, gg.y, gg.z, gg.w};
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                {
-                    const float2 gq = make_float2(gv[q], gv[q]);
-                    e[q][0] = __ffma2_rn(gq, xa, e[q][0]);
-                    e[q][1] = __ffma2_rn(gq, xb, e[q][1]);
+                    const int cell = g4 / a.n4, c4 = g4 - cell * a.n4;
+                    const int src = crow ? crow[cell] : a.cadd[cell * nc + cJ];
+                    cur.off[h] = static_cast<uint32_t>(src * a.n4 + c4) * static_cast<uint32_t>(t1_rows(aI) * bI);
                 }
             }
         };
-        bool ok = true;
-        int st_count = 0;
-        // split E into 3 BF16 pieces and store the 4 x 8 values (jl, column) of j group jh
-        auto store_e = [&](unsigned char *stg, int jh, const float2 (&e)[JH][2]) {
-#pragma unroll
-            for (int jl = 0; jl < JH; ++jl)
+        // copies the next T1_XD rows into the slot before `slot` and moves on (no copy past the last chunk)
+        const uint32_t xdst = smem_u32(xring) + t * 16;
+        auto fetch = [&](int slot) {
+            const uint32_t dst = xdst + (slot == 0 ? T1_XR - 1 : slot - 1) * (T1_XD * 2 * T1_PRODUCERS * 16);
+            if (cur.kc < kc1)
             {
-                uint32_t h01, m01, l01, h23, m23, l23;
-                split3_pair(e[jl][0], h01, m01, l01);
-                split3_pair(e[jl][1], h23, m23, l23);
-                const uint32_t off = sw128_offset(r, (jh * JH + jl) * CW + cq * 4);
-                *reinterpret_cast<uint2 *>(stg + off) = make_uint2(h01, h23);
-                *reinterpret_cast<uint2 *>(stg + A_TILE + off) = make_uint2(m01, m23);
-                *reinterpret_cast<uint2 *>(stg + 2 * A_TILE + off) = make_uint2(l01, l23);
-            }
-        };
-        if constexpr (P2)
-        {
-            // Narrow layout: 2 columns a thread (float2 gathers, one packed FMA per (i, j)).  The
-            // chunk's 2 RA rows (pass, i) are read in the flat order q = pass RA + i, each XD steps
-            // before its use from an XD-entry register ring; the last XD reads of a chunk fetch the
-            // first rows of the next one.  The order is padded to QP, a multiple of XD, so that
-            // row q of every chunk sits in ring slot q mod XD.
-            constexpr int XD = 8;
-            constexpr int QP = (2 * RA + XD - 1) / XD * XD;
-            static_assert(XD <= 2 * RA, "ring deeper than a chunk");
-            const float2 zero2 = make_float2(0.f, 0.f);
-            auto chunk_base = [&](int kc, const float *&b0, const float *&b1) -> bool {
-                const long long col0 = static_cast<long long>(kc) * CW + cq * 2;
-                if (kc >= kc1 || col0 >= nsup || !valid) return false;
-                const int cp = static_cast<int>(col0 / nao), ao = static_cast<int>(col0 % nao);
-                const long long src = static_cast<long long>(a.cadd[cp * nc + cJ]) * nao + ao;
-                b0 = Xp[0] + xrow * nsup + src;
-                b1 = Xp[1] + xrow * nsup + src;
-                return true;
-            };
-            auto ld = [&](const float *b0, const float *b1, int q, bool live) -> float2 {
-                const int i = q % RA;
-                const float *b = q < RA ? b0 : b1;
-                return (live && q < 2 * RA && i < aI) ? __ldg(reinterpret_cast<const float2 *>(b + i * nsup)) : zero2;
-            };
-            const float *c0 = Xp[0], *c1 = Xp[0], *n0 = Xp[0], *n1 = Xp[0];
-            bool clive = chunk_base(kc0, c0, c1);
-            bool nlive = chunk_base(kc0 + 1, n0, n1);
-            float2 xb[XD];
 #pragma unroll
-            for (int q = 0; q < XD; ++q) xb[q] = ld(c0, c1, q, clive);
-            for (int kc = kc0; kc < kc1 && ok; ++kc)
-            {
-                float2 e[4][JH];  // [group of 4 j][jl]: j 0..15, the thread's 2 columns
-#pragma unroll
-                for (int jh = 0; jh < 4; ++jh)
-#pragma unroll
-                    for (int jl = 0; jl < JH; ++jl) e[jh][jl] = zero2;
-#pragma unroll
-                for (int q = 0; q < QP; ++q)
-                {
-                    const int pass = q / RA, i = q % RA;
-                    const float2 x = xb[q % XD];
-                    xb[q % XD] = q + XD < QP ? ld(c0, c1, q + XD, clive) : ld(n0, n1, q + XD - QP, nlive);
-                    if (q >= 2 * RA) continue;  // padding of the read order
-#pragma unroll
-                    for (int jh = 0; jh < 4; ++jh)
-                    {
-                        const float4 gg = gp[pass][(i * gst + jh * JH) / 4];
-                        const float gv[4] = {gg.x, gg.y, gg.z, gg.w};
-#pragma unroll
-                        for (int qq = 0; qq < 4; ++qq)
-                        {
-                            if (RA == 13 && 4 * jh + qq >= 13) continue;
-                            e[jh][qq] = __ffma2_rn(make_float2(gv[qq], gv[qq]), x, e[jh][qq]);
-                        }
-                    }
-                }
-                c0 = n0;
-                c1 = n1;
-                clive = nlive;
-                nlive = chunk_base(kc + 2, n0, n1);
-#pragma unroll
-                for (int jg = 0; jg < 2; ++jg)
-                {
-                    if (jg >= njg || !ok) break;
-                    const int s = st_count % T1_STAGES, rr = st_count / T1_STAGES;
-                    ++st_count;
-                    unsigned char *stg = smem + s * stage_bytes;
-                    if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], (rr & 1) ^ 1)))
-                    {
-                        if (lane == 0) atomicExch(a.err, 201);
-                        ok = false;
-                        break;
-                    }
-#pragma unroll
-                    for (int jh = 0; jh < 2; ++jh)
-#pragma unroll
-                        for (int jl = 0; jl < JH; ++jl)
-                        {
-                            uint32_t h, m, l;
-                            split3_pair(e[2 * jg + jh][jl], h, m, l);
-                            const uint32_t off = sw128_offset(r, (jh * JH + jl) * CW + cq * 2);
-                            *reinterpret_cast<uint32_t *>(stg + off) = h;
-                            *reinterpret_cast<uint32_t *>(stg + A_TILE + off) = m;
-                            *reinterpret_cast<uint32_t *>(stg + 2 * A_TILE + off) = l;
-                        }
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&full[s]);
-                }
-            }
-        }
-        else if constexpr (STREAM)
-        {
-            // One chunk (both stages, all 16 j) per pass over its 2 RA rows (pass, i) of X.
-            // Row (pass, i) of chunk kc sits in xb[i] from RA steps before its use: reading
-            // pass 0 row i refills xb[i] with pass 1 row i, reading pass 1 row i refills it
-            // with pass 0 row i of chunk kc + 1, so the gathers stay half a chunk ahead.
-            const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            auto chunk_base = [&](int kc, const float *&b0, const float *&b1) -> bool {
-                const long long col0 = static_cast<long long>(kc) * CW + cq * 4;
-                if (kc >= kc1 || col0 >= nsup || !valid) return false;
-                const int cp = static_cast<int>(col0 / nao), ao = static_cast<int>(col0 % nao);
-                const long long src = static_cast<long long>(a.cadd[cp * nc + cJ]) * nao + ao;
-                b0 = Xp[0] + xrow * nsup + src;
-                b1 = Xp[1] + xrow * nsup + src;
-                return true;
-            };
-            auto ld = [&](const float *b, int i, bool live) -> float4 {
-                return (live && i < aI) ? __ldg(reinterpret_cast<const float4 *>(b + i * nsup)) : zero4;
-            };
-            const float *c0 = Xp[0], *c1 = Xp[0], *n0 = Xp[0], *n1 = Xp[0];
-            bool clive = chunk_base(kc0, c0, c1);
-            bool nlive = chunk_base(kc0 + 1, n0, n1);
-            float4 xb[RA];
-#pragma unroll
-            for (int i = 0; i < RA; ++i) xb[i] = ld(c0, i, clive);
-            for (int kc = kc0; kc < kc1 && ok; ++kc)
-            {
-                float2 e[4][JH][2];  // [group of 4 j][jl][column pair]: j 0..15
-#pragma unroll
-                for (int jh = 0; jh < 4; ++jh)
-#pragma unroll
-                    for (int jl = 0; jl < JH; ++jl) e[jh][jl][0] = e[jh][jl][1] = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int pass = 0; pass < 2; ++pass)
-                {
-#pragma unroll
-                    for (int i = 0; i < RA; ++i)
-                    {
-                        const float4 x = xb[i];
-                        xb[i] = pass == 0 ? ld(c1, i, clive) : ld(n0, i, nlive);
-                        const float2 xa = make_float2(x.x, x.y), xc = make_float2(x.z, x.w);
-#pragma unroll
-                        for (int jh = 0; jh < 4; ++jh)
-                        {
-                            const float4 gg = gp[pass][(i * gst + jh * JH) / 4];
-                            const float gv[4] = {gg.x, gg.y, gg.z, gg.w};
-#pragma unroll
-                            for (int q = 0; q < 4; ++q)
-                            {
-                                // RA = 13: no atom has more than 13 NAOs, j = 13..15 stay zero
-                                if (RA == 13 && 4 * jh + q >= 13) continue;
-                                const float2 gq = make_float2(gv[q], gv[q]);
-                                e[jh][q][0] = __ffma2_rn(gq, xa, e[jh][q][0]);
-                                e[jh][q][1] = __ffma2_rn(gq, xc, e[jh][q][1]);
-                            }
-                        }
-                    }
-                }
-                c0 = n0;
-                c1 = n1;
-                clive = nlive;
-                nlive = chunk_base(kc + 2, n0, n1);
-                // stage (kc, jg) holds j [8 jg, 8 jg + 8): the groups of 4 j are 2 jg and 2 jg + 1
-#pragma unroll
-                for (int jg = 0; jg < 2; ++jg)
-                {
-                    if (jg >= njg || !ok) break;
-                    const int s = st_count % T1_STAGES, rr = st_count / T1_STAGES;
-                    ++st_count;
-                    unsigned char *stg = smem + s * stage_bytes;
-                    if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], (rr & 1) ^ 1)))
-                    {
-                        if (lane == 0) atomicExch(a.err, 201);
-                        ok = false;
-                        break;
-                    }
-                    store_e(stg, 0, e[2 * jg]);
-                    store_e(stg, 1, e[2 * jg + 1]);
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&full[s]);
-                }
-            }
-        }
-        else
-        {
-        float4 x0[RA], x1[BOTHX ? RA : 1];
-        for (int kc = kc0; kc < kc1 && ok; ++kc)
-        {
-            if constexpr (BOTHX) load_x(kc, 0, 2, x0, x1);
-            for (int jg = 0; jg < njg; ++jg, ++st_count)
-            {
-                const int s = st_count % T1_STAGES, rr = st_count / T1_STAGES;
-                unsigned char *stg = smem + s * stage_bytes;
-#pragma unroll 1
                 for (int h = 0; h < 2; ++h)
                 {
-                    const int j0 = jg * JG + h * JH;
-                    float2 e[JH][2];
+                    const bool live = cur.live[h] && cur.q < t1_rows(aI);  // a multiple of T1_XD
+                    const float4 *src = xrow + (live ? cur.off[h] + static_cast<uint32_t>(cur.q * bI) : 0u);
+                    const int d = live ? bI : 0;
 #pragma unroll
-                    for (int jl = 0; jl < JH; ++jl) e[jl][0] = e[jl][1] = make_float2(0.f, 0.f);
-                    if constexpr (BOTHX)
-                    {
-                        contract(gp[0], j0, x0, e);
-                        contract(gp[1], j0, x1, e);
-                    }
-                    else
-                    {
-                        load_x(kc, 0, 1, x0, x1);
-                        contract(gp[0], j0, x0, e);
-                        load_x(kc, 1, 1, x0, x1);
-                        contract(gp[1], j0, x0, e);
-                    }
-                    if (h == 0)
-                    {
-                        // warp-uniform outcome: the warp arrives on full[s] as one
-                        if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], (rr & 1) ^ 1)))
-                        {
-                            if (lane == 0) atomicExch(a.err, 201);
-                            ok = false;
-                            break;
-                        }
-                    }
-#pragma unroll
-                    for (int jl = 0; jl < JH; ++jl)
-                    {
-                        uint32_t h01, m01, l01, h23, m23, l23;
-                        split3_pair(e[jl][0], h01, m01, l01);
-                        split3_pair(e[jl][1], h23, m23, l23);
-                        const uint32_t off = sw128_offset(r, (h * JH + jl) * CW + cq * 4);
-                        *reinterpret_cast<uint2 *>(stg + off) = make_uint2(h01, h23);
-                        *reinterpret_cast<uint2 *>(stg + A_TILE + off) = make_uint2(m01, m23);
-                        *reinterpret_cast<uint2 *>(stg + 2 * A_TILE + off) = make_uint2(l01, l23);
-                    }
+                    for (int u = 0; u < T1_XD; ++u) cp_async16(dst + (2 * u + h) * T1_PRODUCERS * 16, src + u * d, live);
                 }
-                if (!ok) break;
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full[s]);
+                cur.q += T1_XD;
+                if (cur.q >= nq)
+                {
+                    cur.q = 0;
+                    if (++cur.un == nunit) point_at(cur.kc + 2);
+                }
+            }
+            cp_async_commit();
+        };
+        const uint32_t atile = tmem + (static_cast<uint32_t>((warp % 4) * 32) << 16) + T1_ABASE + set * T1_ACOLS;
+        point_at(kc0 + set);
+        for (int k = 1; k < T1_XR; ++k) fetch(k);
+        int slot = 0;
+        const uint32_t xown = smem_u32(xring) + t * 16;
+        uint32_t use = 3u;  // bit h: phase to wait for before half h of the A tile is written again
+        bool ok = true;
+        for (int kc = kc0 + set; kc < kc1 && ok; kc += 2)
+        {
+            for (int un = 0; un < nunit && ok; ++un)
+            {
+                const int nj = wide ? aJ : min(JG, aJ - un * JG);
+                const uint32_t gu = gs + un * (gq * JG * 4);
+#define GB_T1_UNIT(NJ) \
+    ok = t1_unit<NJ>(xown, slot, fetch, gu, gq, nq, (nj + 3) / 4, atile, full + 2 * set, empty + 2 * set, use, lane, a.err)
+                // as many registers of E as j, by half stages of 4
+                if (nj <= 2) GB_T1_UNIT(2);
+                else if (nj <= 4) GB_T1_UNIT(4);
+                else if (nj <= 5) GB_T1_UNIT(5);
+                else if (nj <= 8) GB_T1_UNIT(8);
+                else if constexpr (JT == 16)
+                {
+                    if (nj <= 10) GB_T1_UNIT(10);
+                    else if (nj <= 12) GB_T1_UNIT(12);
+                    else if (nj <= 13) GB_T1_UNIT(13);
+                    else GB_T1_UNIT(14);
+                }
+#undef GB_T1_UNIT
             }
         }
+        cp_async_wait<0>();
     }
+    else if (warp >= T1_ISSUE)
+    {
+        // ---------------- issue warp: per stage st, the MMAs of st and the C^J copy of st + nbs - 1
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CREG));
+        if (warp == T1_ISSUE)  // the whole warp, converged: one elected lane issues
+        {
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint32_t bbytes = static_cast<uint32_t>(NT) * 64 * 2;  // one piece of a B tile
+            const int sp = a.spec[J], zj = a.spec_idx[J];
+            const long long ktot = maps.ktot[sp];
+            // C^J tiles stream through L2 once per tile: evict them first, keep the X^I rows
+            const uint64_t pol_b = l2_policy_evict_first();
+            int ts = 0, tph = 1, copied = 0;  // B ring: next stage to fill
+            auto issue_tma = [&]() -> bool {
+                if (!__all_sync(0xffffffffu, mbar_wait_nap<20>(&bempty[ts], tph)))
+                {
+                    if (lane == 0) atomicExch(a.err, 202);
+                    return false;
+                }
+                const int x = (kc0 * njg + copied) * 64;  // K offset (kc * njg + jg) * 64
+                if (x < 0 || static_cast<long long>(x) + 64 > ktot || (x & 7) != 0)
+                {
+                    if (lane == 0) atomicExch(a.err, 205);  // coordinate outside the C^J operand: skip the copy
+                    return false;
+                }
+                unsigned char *bst = bring + ts * bstage_bytes;
+                if (elect_one())
+                {
+                    mbar_arrive_expect_tx(&bfull[ts], NS * bbytes);
+#pragma unroll
+                    for (int p = 0; p < NS; ++p)  // pieces stacked along N: rows [p NT, (p + 1) NT)
+                        tma_load_3d_hint(bst + p * bbytes, &maps.m[sp][p], x, 0, zj, &bfull[ts], pol_b);
+                }
+                __syncwarp();
+                ++copied;
+                if (++ts == nbs) ts = 0, tph ^= 1;
+                return true;
+            };
+            bool ok = true;
+            for (int st = 0; st < nbs - 1 && st < total_stages && ok; ++st) ok = issue_tma();
+            int sb = 0, pb = 0, ab = 0, pa = 1, jg = 0, set = 0;
+            uint32_t pf = 0;  // bit 2 set + half: phase of that half of the warpgroup's A tile
+            const int nhalf = (aJ + 3) / 4;  // half stages of a chunk
+            for (int st = 0; st < total_stages && ok; ++st)
+            {
+                unsigned char *bst = bring + sb * bstage_bytes;
+                const uint32_t tb = tm + static_cast<uint32_t>(ab * NBLK * NT);
+                const uint64_t db0 = smem_desc_sw128(bst);
+                const int nh = min(2, nhalf - 2 * jg);
+                for (int h = 0; h < nh && ok; ++h)
+                {
+                    const int fb = 2 * set + h;
+                    if (!__all_sync(0xffffffffu, mbar_wait_nap<50>(&full[fb], (pf >> fb) & 1) &&
+                                                     (h != 0 || (mbar_wait_nap<20>(&bfull[sb], pb) &&
+                                                                 mbar_wait_nap<20>(&acce[ab], pa)))))
+                    {
+                        if (lane == 0) atomicExch(a.err, 203);
+                        ok = false;
+                        break;
+                    }
+                    pf ^= 1u << fb;
+                    tc_fence_after();
+                    const uint32_t ta = tm + T1_ABASE + set * T1_ACOLS + h * 16;
+                    const uint64_t db = db0 + static_cast<uint64_t>(h * 64 >> 4);
+                    if (elect_one())
+                    {
+                        if constexpr (STACKN)
+                        {
+                            const uint32_t i3 = idesc_bf16_f32(T1_BM, 3 * NT), i2 = idesc_bf16_f32(T1_BM, 2 * NT),
+                                           i1 = idesc_bf16_f32(T1_BM, NT);
+#pragma unroll
+                            for (int k = 0; k < 2; ++k)  // hi x [Ch;Cm;Cl]
+                                mma_bf16_ta(tb, ta + k * 8, db + 2 * k, i3, (h | k) != 0);
+#pragma unroll
+                            for (int k = 0; k < 2; ++k)  // mid x [Ch;Cm]
+                                mma_bf16_ta(tb + NT, ta + 32 + k * 8, db + 2 * k, i2, 1);
+#pragma unroll
+                            for (int k = 0; k < 2; ++k)  // lo x Ch
+                                mma_bf16_ta(tb + 2 * NT, ta + 64 + k * 8, db + 2 * k, i1, 1);
+                        }
+                        else
+                        {
+                            const uint32_t idesc = idesc_bf16_f32(T1_BM, NT);
+                            const uint32_t t_hh = tb, t_x = tb + NT;
+                            const uint64_t dp = static_cast<uint64_t>(bbytes >> 4);  // to the next piece of C^J
+#pragma unroll
+                            for (int k = 0; k < 2; ++k)
+                            {
+                                const uint64_t d0 = db + static_cast<uint64_t>(k * 32 >> 4);
+                                const uint32_t ah = ta + k * 8, am = ah + 32, al = ah + 64;
+                                // cross terms (smallest first) into t_x, hi*hi into t_hh; both restart each stage
+                                mma_bf16_ta(t_x, al, d0, idesc, (h | k) != 0);
+                                mma_bf16_ta(t_x, ah, d0 + 2 * dp, idesc, 1);
+                                mma_bf16_ta(t_x, am, d0 + dp, idesc, 1);
+                                mma_bf16_ta(t_x, am, d0, idesc, 1);
+                                mma_bf16_ta(t_x, ah, d0 + dp, idesc, 1);
+                                mma_bf16_ta(t_hh, ah, d0, idesc, (h | k) != 0);
+                            }
+                        }
+                        mma_commit(&empty[fb]);
+                        if (h == nh - 1)
+                        {
+                            mma_commit(&bempty[sb]);
+                            mma_commit(&accf[ab]);
+                        }
+                    }
+                    __syncwarp();
+                }
+                if (!ok) break;
+                if (++sb == nbs) sb = 0, pb ^= 1;
+                if (++ab == nab) ab = 0, pa ^= 1;
+                if (++jg == njg) jg = 0, set ^= 1;
+                if (copied < total_stages) ok = issue_tma();
+            }
+            // every issued MMA and copy completes before the CTA's TMEM and shared memory are released
+            if (elect_one()) mma_commit(fin);
+            __syncwarp();
+            mbar_wait(fin, 0);
+            for (int k = max(0, copied - nbs); k < copied; ++k) mbar_wait(&bfull[k % nbs], (k / nbs) & 1);
         }
+    }
     else
     {
         // ---------------- drain warps: per-stage accumulator blocks -> FP32 registers -> chi0R.
-        // Lane 0 of warp 8 issues, per stage st, the MMAs of st and then the C^J TMA copy of
-        // st + nbs - 1 (nbs - 1 stages of look-ahead hide the HBM latency of the B tiles),
-        // before its warp drains st - 1: the tensor pipe always holds the next stage.
-        const int wq = warp - DRAIN_WARP0;
-        const bool ctrl = wq == 0 && lane == 0;
+        if constexpr (DREG > 128)
+            asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(DREG));
+        else
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(DREG));
+        const int wq = warp - T1_DRAIN;
         const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
-        const uint32_t bbytes = static_cast<uint32_t>(NT) * 64 * 2;  // one piece of a B tile
-        const int sp = a.spec[J], zj = a.spec_idx[J];
-        const long long ktot = maps.ktot[sp];
-        // C^J tiles stream through L2 once per tile: evict them first, keep the X^I rows
-        const uint64_t pol_b = l2_policy_evict_first();
-        auto issue_tma = [&](int st) -> bool {
-            const int s = st % nbs, rr = st / nbs;
-            if (!mbar_wait(&bempty[s], (rr & 1) ^ 1))
-            {
-                atomicExch(a.err, 202);
-                return false;
-            }
-            const int x = (kc0 * njg + st) * 64;  // K offset (kc * njg + jg) * 64
-            if (x < 0 || static_cast<long long>(x) + 64 > ktot || (x & 7) != 0)
-            {
-                atomicExch(a.err, 205);  // coordinate outside the C^J operand: skip the copy
-                return false;
-            }
-            unsigned char *bst = bring + s * bstage_bytes;
-            mbar_arrive_expect_tx(&bfull[s], NS * bbytes);
+        float2 acc[NTC / 2];
 #pragma unroll
-            for (int p = 0; p < NS; ++p)  // pieces stacked along N: rows [p NT, (p + 1) NT)
-                tma_load_3d_hint(bst + p * bbytes, &maps.m[sp][p], x, 0, zj, &bfull[s], pol_b);
-            return true;
-        };
-        auto issue_mma = [&](int st) -> bool {
-            const int s = st % T1_STAGES, rr = st / T1_STAGES;
-            const int sb = st % nbs, rb = st / nbs;
-            const int ab = st & 1;
-            if (!mbar_wait(&full[s], rr & 1) || !mbar_wait(&bfull[sb], rb & 1) ||
-                !mbar_wait(&acce[ab], ((st >> 1) & 1) ^ 1))
-            {
-                atomicExch(a.err, 203);
-                return false;
-            }
-            tc_fence_after();
-            unsigned char *stg = smem + s * stage_bytes;
-            unsigned char *bst = bring + sb * bstage_bytes;
-            const uint32_t tb = tmem + static_cast<uint32_t>(ab * NBLK * NTC);
-            uint64_t da[NS], db[NS];
-#pragma unroll
-            for (int p = 0; p < NS; ++p)
-            {
-                da[p] = smem_desc_sw128(stg + p * A_TILE);
-                db[p] = smem_desc_sw128(bst + p * bbytes);
-            }
-            if constexpr (STACKN)
-            {
-                const uint32_t i3 = idesc_bf16_f32(T1_BM, 3 * NT), i2 = idesc_bf16_f32(T1_BM, 2 * NT),
-                               i1 = idesc_bf16_f32(T1_BM, NT);
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                {
-                    const uint64_t dk = static_cast<uint64_t>(k * 32 >> 4);
-                    mma_bf16(tb, da[0] + dk, db[0] + dk, i3, k != 0);                       // hi x [Ch;Cm;Cl]
-                    mma_bf16(tb + NT, da[1] + dk, db[0] + dk, i2, 1);                       // mid x [Ch;Cm]
-                    mma_bf16(tb + 2 * NT, da[2] + dk, db[0] + dk, i1, 1);                   // lo x Ch
-                }
-            }
-            else
-            {
-                const uint32_t idesc = idesc_bf16_f32(T1_BM, NT);
-                const uint32_t t_hh = tb, t_x = tb + NTC;
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                {
-                    const uint64_t dk = static_cast<uint64_t>(k * 32 >> 4);
-                    // cross terms (smallest first) into t_x, hi*hi into t_hh; both restart each stage
-                    mma_bf16(t_x, da[2] + dk, db[0] + dk, idesc, k != 0);
-                    mma_bf16(t_x, da[0] + dk, db[2] + dk, idesc, 1);
-                    mma_bf16(t_x, da[1] + dk, db[1] + dk, idesc, 1);
-                    mma_bf16(t_x, da[1] + dk, db[0] + dk, idesc, 1);
-                    mma_bf16(t_x, da[0] + dk, db[1] + dk, idesc, 1);
-                    mma_bf16(t_hh, da[0] + dk, db[0] + dk, idesc, k != 0);
-                }
-            }
-            mma_commit(&empty[s]);
-            mma_commit(&bempty[sb]);
-            mma_commit(&accf[ab]);
-            return true;
-        };
-        float acc[NTC];
-#pragma unroll
-        for (int c = 0; c < NTC; ++c) acc[c] = 0.0f;
+        for (int c = 0; c < NTC / 2; ++c) acc[c] = make_float2(0.f, 0.f);
+        auto pair_of = [](const uint32_t *r, int i) { return make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])); };
         bool ok = true;
-        int issued = 0, copied = 0;  // MMA stages and B-tile copies issued (control lane)
-        if (ctrl)
-            for (int st = 0; st < nbs - 1 && st < total_stages && ok; ++st)
-                if ((ok = issue_tma(st))) ++copied;
-        for (int st = 0; st <= total_stages; ++st)
+        int ab = 0, ph = 0;
+        for (int sd = 0; sd < total_stages; ++sd)
         {
-            if (wq == 0)
+            // one warp polls; the others stand at the barrier
+            if (wq == 0 && !__all_sync(0xffffffffu, mbar_wait_nap<100>(&accf[ab], ph)) && lane == 0)
             {
-                if (ctrl && ok && st < total_stages)
-                {
-                    ok = issue_mma(st);
-                    if (ok) ++issued;
-                    if (ok && st + nbs - 1 < total_stages)
-                        if ((ok = issue_tma(st + nbs - 1))) ++copied;
-                }
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                atomicExch(a.err, 204);
+                *drain_stop = 1;
             }
-            if (!ok) break;
-            if (st == 0) continue;
-            const int sd = st - 1, ab = sd & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait(&accf[ab], (sd >> 1) & 1)))
+            named_bar_sync(2, 128);
+            if (*drain_stop)
             {
-                if (lane == 0) atomicExch(a.err, 204);
                 ok = false;
                 break;
             }
             tc_fence_after();
-            const uint32_t tb = tmem + static_cast<uint32_t>(ab * NBLK * NTC) + lane_base;
+            const uint32_t tb = tmem + static_cast<uint32_t>(ab * NBLK * NT) + lane_base;
 #pragma unroll
-            for (int c0 = 0; c0 < NTC; c0 += 16)
+            for (int c0 = 0; c0 < NTC; c0 += 8)
             {
                 if (c0 < NT)
                 {
-                    if constexpr (STACKN && P2)
+                    // 8 columns of each block live at a time, added from the smallest order up
+                    uint32_t v[8], u[8];
+                    tmem_ld8_nowait(tb + (NBLK - 1) * NT + c0, v);
+                    if constexpr (STACKN)
                     {
-                        // narrow layout (96 registers a thread): one block of 16 loaded values live
-                        // at a time, added into the running sums from the leading block down
-#pragma unroll
-                        for (int b = 0; b < 3; ++b)
-                        {
-                            uint32_t v[16];
-                            tmem_ld16_nowait(tb + b * NT + c0, v);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) acc[c0 + i] += __uint_as_float(v[i]);
-                        }
-                    }
-                    else if constexpr (STACKN)
-                    {
-                        uint32_t v0[16], v1[16], v2[16];
-                        tmem_ld16_nowait(tb + c0, v0);
-                        tmem_ld16_nowait(tb + NT + c0, v1);
-                        tmem_ld16_nowait(tb + 2 * NT + c0, v2);
+                        uint32_t m[8];
+                        tmem_ld8_nowait(tb + NT + c0, m);
+                        tmem_ld8_nowait(tb + c0, u);
                         tmem_wait_ld();
 #pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            acc[c0 + i] += __uint_as_float(v0[i]) + (__uint_as_float(v1[i]) + __uint_as_float(v2[i]));
+                        for (int i = 0; i < 8; i += 2)
+                            acc[(c0 + i) / 2] = __fadd2_rn(acc[(c0 + i) / 2],
+                                                           __fadd2_rn(pair_of(u, i), __fadd2_rn(pair_of(m, i), pair_of(v, i))));
                     }
                     else
                     {
-                        uint32_t vx[16], vh[16];
-                        tmem_ld16_nowait(tb + NTC + c0, vx);
-                        tmem_ld16_nowait(tb + c0, vh);
+                        tmem_ld8_nowait(tb + c0, u);
                         tmem_wait_ld();
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) acc[c0 + i] += __uint_as_float(vx[i]);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) acc[c0 + i] += __uint_as_float(vh[i]);
+                        for (int i = 0; i < 8; i += 2)
+                            acc[(c0 + i) / 2] =
+                                __fadd2_rn(__fadd2_rn(acc[(c0 + i) / 2], pair_of(v, i)), pair_of(u, i));
                     }
                 }
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acce[ab]);
+            if (++ab == nab) ab = 0, ph ^= 1;
         }
-        if (ctrl && !ok && issued > 0)
-        {
-            // error path: let this CTA's issued MMAs finish before its TMEM is released
-            const int last = issued - 1;
-            mbar_wait(&empty[last % T1_STAGES], (last / T1_STAGES) & 1);
-        }
-        if (ctrl && !ok)
-            for (int st = issued; st < copied; ++st)  // and its B copies land before the CTA exits
-                mbar_wait(&bfull[st % nbs], (st / nbs) & 1);
         int grp = 0, mu = 0;
         if (ok && row_of(wq * 32 + lane, grp, mu))
         {
@@ -792,99 +708,109 @@ __global__ void __launch_bounds__(T1Layout<P2>::threads, 1) k_t1_tc(const __grid
             for (int c = 0; c < NTC; ++c)
                 if (c < bJ)
                 {
+                    const double v = static_cast<double>(c & 1 ? acc[c / 2].y : acc[c / 2].x);
                     if (w.split)
-                        atomicAdd(orow + c, static_cast<double>(acc[c]));
+                        atomicAdd(orow + c, v);
                     else
-                        orow[c] = static_cast<double>(acc[c]);
+                        orow[c] = v;
                 }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
+    if (warp == 0) tmem_dealloc(tmem, T1_TMEM);
 }
 
 // T2 for one (pair, cJ) and one 64 x 64 tile of its (mu, nu) block:
 //   out[mu][nu] += sum_pass sum_{i,j} Xb^I[mu i; (cJ,J) j] * Xa^J[nu j; (-cJ,I) i].
-// Grid: x = (pair, cJ) group, y = output tile (T2_TILES x T2_TILES of them; CTAs beyond the
-// pair's own block return at once), so that a Gamma-only cell, with one group per pair, still
-// spreads over the SMs.  Per pass and chunk of i, the two operands are staged K-major in
-// shared memory (K = (i, j)): S1[k][mu] and S2[k][nu]; each of the 256 threads accumulates a
-// 4 x 4 block of (mu, nu) with two 16-byte shared loads per 16 FMAs.  Tiles are disjoint and the
-// CTA sums both passes before its one add, so the result does not depend on CTA order.
+// Grid: x = (pair, cJ) group, y = output tile (CTAs beyond the pair's own block return at once), so that a
+// Gamma-only cell, with one group per pair, still spreads over the SMs.  Both operands come from the
+// 4-column groups of Xt: a float4 is 4 j of one (mu, i) or 4 i of one (nu, j), and 32 lanes read 512
+// contiguous bytes.  A step takes 4 i x 4 j: one float4 of each operand per thread, transposed through
+// shared memory to [k = (i, j)][mu] and [k][nu] without bank conflicts, the next step's loads in flight
+// meanwhile; each of the tile's (mu, nu) 4 x 4 blocks is one thread's.  Bound by the latency of its steps
+// in small cells and by the FP32 pipe in large ones.  Tiles are disjoint and the CTA sums both passes
+// before its one add, so the result does not depend on CTA order.
 constexpr int T2_THREADS = 256;
 constexpr int T2_TILE = 64;
-constexpr int T2_TILES = T1_NMAX / T2_TILE;  // per dimension: up to 128 ABFs per atom
-constexpr int T2_SMEM_FLOATS = 12288;        // 48 KB
 
-__global__ void __launch_bounds__(T2_THREADS) k_t2(const float *__restrict__ X, long long xsign, Geom g, Pairs pr,
-                                                  const T1Group *__restrict__ groups, double *__restrict__ out)
+__global__ void __launch_bounds__(T2_THREADS) k_t2(const float4 *__restrict__ Xt, const long long *__restrict__ xoff, int n4,
+                                                  Geom g, Pairs pr, const T1Group *__restrict__ groups, int tiles,
+                                                  double *__restrict__ out)
 {
-    __shared__ __align__(16) float sm[T2_SMEM_FLOATS];
+    __shared__ __align__(16) float S1[2][16][T2_TILE], S2[2][16][T2_TILE];
     const int p = groups[blockIdx.x].pair, cJ = groups[blockIdx.x].cell;
     const int I = pr.I[p], J = pr.J[p];
     const int aI = g.nao[I], aJ = g.nao[J], bI = g.nabf[I], bJ = g.nabf[J];
-    const int mt0 = static_cast<int>(blockIdx.y / T2_TILES) * T2_TILE, nt0 = static_cast<int>(blockIdx.y % T2_TILES) * T2_TILE;
+    const int mt0 = static_cast<int>(blockIdx.y) / tiles * T2_TILE, nt0 = static_cast<int>(blockIdx.y) % tiles * T2_TILE;
     if (mt0 >= bI || nt0 >= bJ) return;  // whole CTA: no barrier skipped by part of it
     const int mn = min(T2_TILE, bI - mt0), nn = min(T2_TILE, bJ - nt0);
-    const long long nsup = g.n_sup;
-    const long long colJ = static_cast<long long>(cJ) * g.n_ao + g.ao_off[J];
-    const long long colI = static_cast<long long>(g.cneg[cJ]) * g.n_ao + g.ao_off[I];
-    double *o = out + pr.r_off[p] + static_cast<long long>(cJ) * bI * bJ;
-    // i per chunk so that both operands fit: 2 * T2_TILE * ic * aJ floats
-    const int ic = max(1, min(aI, T2_SMEM_FLOATS / (2 * T2_TILE * aJ)));
-    float *S1 = sm;                                                // [k][T2_TILE]
-    float *S2 = sm + static_cast<size_t>(ic) * aJ * T2_TILE;       // [k][T2_TILE]
-    const int m0 = (static_cast<int>(threadIdx.x) / (T2_TILE / 4)) * 4;
-    const int n0 = (static_cast<int>(threadIdx.x) % (T2_TILE / 4)) * 4;
-    float acc[4][4];
+    // first column group of each atom and the atom's first column inside it
+    const int gI = g.ao_off[I] / 4, sI = g.ao_off[I] % 4, gJ = g.ao_off[J] / 4, sJ = g.ao_off[J] % 4;
+    const int nI = (sI + aI + 3) / 4, nJ = (sJ + aJ + 3) / 4, steps = 2 * nI * nJ;
+    const int r = threadIdx.x % T2_TILE, s = threadIdx.x / T2_TILE;  // staging: row and i (or j) of the step
+    const long long rI = static_cast<long long>(t1_rows(aI)) * bI, rJ = static_cast<long long>(t1_rows(aJ)) * bJ;
+    const float4 *XI = Xt + xoff[I] + (static_cast<long long>(cJ) * n4 + gJ) * rI + mt0 + r;
+    const float4 *XJ = Xt + xoff[J] + (static_cast<long long>(g.cneg[cJ]) * n4 + gI) * rJ + nt0 + r;
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto load = [&](int st, float4 &v1, float4 &v2) {
+        const int pass = st / (nI * nJ), ig = st / nJ % nI, jg = st % nJ;
+        const int i = 4 * ig + s - sI, j = 4 * jg + s - sJ;
+        // pass 0 contracts X(-) of I with X(+) of J, pass 1 the other way round
+        v1 = i >= 0 && i < aI && r < mn ? XI[jg * rI + static_cast<long long>(pass * aI + i) * bI] : zero4;
+        v2 = j >= 0 && j < aJ && r < nn ? XJ[ig * rJ + static_cast<long long>((1 - pass) * aJ + j) * bJ] : zero4;
+    };
+    // one 4 x 4 block of the tile per thread
+    const int nb = (nn + 3) / 4;
+    const int m0 = static_cast<int>(threadIdx.x) / nb * 4, n0 = static_cast<int>(threadIdx.x) % nb * 4;
+    const bool live = m0 < mn;
+    float2 acc[4][2];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
-    for (int pass = 0; pass < 2; ++pass)
+    for (int a = 0; a < 4; ++a) acc[a][0] = acc[a][1] = make_float2(0.f, 0.f);
+    float4 v1, v2;
+    load(0, v1, v2);
+    for (int st = 0; st < steps; ++st)
     {
-        const float *Xb = X + (pass == 0 ? xsign : 0);
-        const float *Xa = X + (pass == 0 ? 0 : xsign);
-        for (int i0 = 0; i0 < aI; i0 += ic)
+        float(*A)[T2_TILE] = S1[st & 1], (*B)[T2_TILE] = S2[st & 1];
+        A[4 * s][r] = v1.x, A[4 * s + 1][r] = v1.y, A[4 * s + 2][r] = v1.z, A[4 * s + 3][r] = v1.w;
+        B[s][r] = v2.x, B[4 + s][r] = v2.y, B[8 + s][r] = v2.z, B[12 + s][r] = v2.w;
+        __syncthreads();
+        if (st + 1 < steps) load(st + 1, v1, v2);
+        if (live)
         {
-            const int ni = min(ic, aI - i0), nk = ni * aJ;
-            __syncthreads();
-            // S1[(i - i0) aJ + j][mu] = Xb[(I, mt0 + mu, i)][(cJ, J, j)]  (j fastest: contiguous reads)
-            for (int t = threadIdx.x; t < T2_TILE * nk; t += T2_THREADS)
-            {
-                const int mu = t / nk, k = t % nk, il = k / aJ, jj = k % aJ;
-                S1[k * T2_TILE + mu] =
-                    mu < mn ? Xb[(g.rowc_off[I] + static_cast<long long>(mt0 + mu) * aI + i0 + il) * nsup + colJ + jj]
-                            : 0.f;
-            }
-            // S2[(i - i0) aJ + j][nu] = Xa[(J, nt0 + nu, j)][(-cJ, I, i)]  (i fastest)
-            for (int t = threadIdx.x; t < T2_TILE * nk; t += T2_THREADS)
-            {
-                const int nu = t / nk, r = t % nk, jj = r / ni, il = r % ni;
-                S2[(il * aJ + jj) * T2_TILE + nu] =
-                    nu < nn ? Xa[(g.rowc_off[J] + static_cast<long long>(nt0 + nu) * aJ + jj) * nsup + colI + i0 + il]
-                            : 0.f;
-            }
-            __syncthreads();
-            for (int k = 0; k < nk; ++k)
-            {
-                const float4 av = *reinterpret_cast<const float4 *>(S1 + k * T2_TILE + m0);
-                const float4 bv = *reinterpret_cast<const float4 *>(S2 + k * T2_TILE + n0);
-                const float a4[4] = {av.x, av.y, av.z, av.w}, b4[4] = {bv.x, bv.y, bv.z, bv.w};
+            // the i and j of this step that lie inside the atoms
+            const int ig = st / nJ % nI, jg = st % nJ;
+            const int i0 = max(0, sI - 4 * ig), i1 = min(4, sI + aI - 4 * ig), j0 = max(0, sJ - 4 * jg),
+                      j1 = min(4, sJ + aJ - 4 * jg);
+            for (int i = i0; i < i1; ++i)
 #pragma unroll
-                for (int a = 0; a < 4; ++a)
+                for (int j = 0; j < 4; ++j)
+                {
+                    if (j < j0 || j >= j1) continue;
+                    const float4 av = *reinterpret_cast<const float4 *>(&A[4 * i + j][m0]);
+                    const float4 bv = *reinterpret_cast<const float4 *>(&B[4 * i + j][n0]);
+                    const float a4[4] = {av.x, av.y, av.z, av.w};
+                    const float2 b0 = make_float2(bv.x, bv.y), b1 = make_float2(bv.z, bv.w);
 #pragma unroll
-                    for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(a4[a], b4[b], acc[a][b]);
-            }
+                    for (int a = 0; a < 4; ++a)
+                    {
+                        const float2 aa = make_float2(a4[a], a4[a]);
+                        acc[a][0] = __ffma2_rn(aa, b0, acc[a][0]);
+                        acc[a][1] = __ffma2_rn(aa, b1, acc[a][1]);
+                    }
+                }
         }
     }
+    if (!live) return;
+    double *o = out + pr.r_off[p] + static_cast<long long>(cJ) * bI * bJ + static_cast<long long>(mt0 + m0) * bJ + nt0 + n0;
 #pragma unroll
     for (int a = 0; a < 4; ++a)
+    {
+        const float v[4] = {acc[a][0].x, acc[a][0].y, acc[a][1].x, acc[a][1].y};
 #pragma unroll
-        for (int b = 0; b < 4; ++b)
-            if (m0 + a < mn && n0 + b < nn)
-                o[static_cast<long long>(mt0 + m0 + a) * bJ + nt0 + n0 + b] += static_cast<double>(acc[a][b]);
+        for (int c = 0; c < 4; ++c)
+            if (m0 + a < mn && n0 + c < nn) o[static_cast<long long>(a) * bJ + c] += static_cast<double>(v[c]);
+    }
 }
 
 // B operand of X = C * Gs: row n = (cL, l), column k = (cK, k'):  Gs^T[n][k] = G[cdiff(cL,cK)][k'][l]
@@ -917,9 +843,50 @@ __global__ void k_gsT_split(const double *__restrict__ G, Geom g, long long kpad
     }
 }
 
-// T1 B-operand layout of atom J: row nu, K index ((kc * aJpad + j) * CW + col) for
-// C^J[nu][j][kc*CW + col] (zero beyond the atom's NAOs and the supercell width).
-__global__ void k_cb_layout(const double *__restrict__ C, Geom g, int J, int ajp, int nkc, long long ktot,
+// X in the order the T1 producers read it: groups of 4 columns of one cell (n4 = ceil(n_ao / 4) per
+// cell, zero past n_ao), atom-major,
+//   Xt[xoff[I] + (g4 t1_rows(a_I) + q) b_I + mu] = the 4 columns of X_b[(I, mu, i)], q = (pass, i),
+// pass 0 of X(-), pass 1 of X(+), zero rows past 2 a_I.  A warp of producers (32 consecutive rows mu)
+// then reads 512 contiguous bytes per q, where row-major X costs it 32 lines.  Grid: x = blocks of 8
+// groups, y = atoms times 32-row tiles of mu, z = blocks of T1_XD rows q; bound by HBM (X read and written once, 1% of the
+// contraction's time).
+__global__ void __launch_bounds__(256) k_x_layout(const float *__restrict__ X, long long xsign, Geom g, int n4, int ng4,
+                                                  int mu_tiles, const long long *__restrict__ xoff,
+                                                  float4 *__restrict__ Xt)
+{
+    __shared__ float tile[T1_XD][32][33];
+    const int I = blockIdx.y / mu_tiles, mu0 = (blockIdx.y % mu_tiles) * 32;
+    const int aI = g.nao[I], bI = g.nabf[I], rows = t1_rows(aI), q0 = blockIdx.z * T1_XD;
+    if (mu0 >= bI || q0 >= rows) return;
+    const int c = threadIdx.x % 32, r0 = threadIdx.x / 32;
+    // the column this thread reads, and the (mu, group) it writes
+    const int g4r = blockIdx.x * 8 + c / 4;
+    const int ao = (g4r % n4) * 4 + c % 4;
+    const bool live = g4r < ng4 && ao < g.n_ao;
+    const long long col = static_cast<long long>(g4r / n4) * g.n_ao + ao;
+#pragma unroll
+    for (int k = 0; k < T1_XD; ++k)
+    {
+        const int q = q0 + k;
+        const bool lq = live && q < 2 * aI;
+        const float *src = X + (q < aI ? xsign : 0) + (g.rowc_off[I] + q % aI) * static_cast<long long>(g.n_sup) + col;
+#pragma unroll
+        for (int r = 0; r < 32; r += 8)
+            tile[k][r + r0][c] = lq && mu0 + r + r0 < bI ? src[static_cast<long long>(mu0 + r + r0) * aI * g.n_sup] : 0.0f;
+    }
+    __syncthreads();
+    const int g4w = blockIdx.x * 8 + r0;
+    if (g4w >= ng4 || mu0 + c >= bI) return;
+    float4 *dst = Xt + xoff[I] + (static_cast<long long>(g4w) * rows + q0) * bI + mu0 + c;
+#pragma unroll
+    for (int k = 0; k < T1_XD; ++k)
+        dst[static_cast<long long>(k) * bI] = make_float4(tile[k][c][4 * r0], tile[k][c][4 * r0 + 1], tile[k][c][4 * r0 + 2],
+                                                          tile[k][c][4 * r0 + 3]);
+}
+
+// T1 B-operand layout of atom J: row nu, K index ((kc * aJpad + j) * CW + col) for C^J[nu][j][column col
+// of chunk kc] (zero beyond the atom's NAOs, the cell's columns and the supercell).
+__global__ void k_cb_layout(const double *__restrict__ C, Geom g, int J, int ajp, int n4, int ng4, long long ktot,
                             __nv_bfloat16 *__restrict__ p0, __nv_bfloat16 *__restrict__ p1,
                             __nv_bfloat16 *__restrict__ p2)
 {
@@ -933,9 +900,11 @@ __global__ void k_cb_layout(const double *__restrict__ C, Geom g, int J, int ajp
         const long long kc = k / (static_cast<long long>(ajp) * CW);
         const int rem = static_cast<int>(k % (static_cast<long long>(ajp) * CW));
         const int j = rem / CW, col = rem % CW;
-        const long long c = kc * CW + col;
+        const int g4 = static_cast<int>(2 * kc + col / 4);
+        const int ao = (g4 % n4) * 4 + col % 4;
         double x = 0.0;
-        if (j < aJ && c < g.n_sup) x = C[(g.rowc_off[J] + static_cast<long long>(nu) * aJ + j) * g.n_sup + c];
+        if (j < aJ && g4 < ng4 && ao < g.n_ao)
+            x = C[(g.rowc_off[J] + static_cast<long long>(nu) * aJ + j) * g.n_sup + static_cast<long long>(g4 / n4) * g.n_ao + ao];
         const __nv_bfloat16 h = __double2bfloat16(x);
         const double r1 = x - static_cast<double>(__bfloat162float(h));
         const __nv_bfloat16 m = __double2bfloat16(r1);
@@ -953,11 +922,13 @@ struct TcChi0::Impl
     Geom g;
     Pairs pr;
     long long kpad = 0;
-    int nkc = 0;
+    int nkc = 0, n4 = 0, ng4 = 0;
     bool t1_simt = false;
     SplitStore csplit, gs;
     DevBuf<float> X, Gf, Cf;
-    DevBuf<int> err, cadd, ajpad;
+    DevBuf<float4> Xt;
+    DevBuf<long long> xoff;
+    DevBuf<int> err, cadd;
     DevBuf<T1Work> work;
     DevBuf<T1Group> groups;
     int n_work = 0, n_groups = 0;
@@ -971,14 +942,13 @@ struct TcChi0::Impl
     std::vector<SplitStore> cb;  // per species: C^J of its atoms, stacked
     T1Maps maps{};
     DevBuf<int> spec, spec_idx;
-    int b_tile = 0, maxcj = 0, smem = 0, ra = 16, ntc = 64, nbs = 2, gj = JG;
-    // Launch choices of the contraction: producer layout and K parts per tile.  The tuner
-    // times the candidates on the first unscreened contraction of a shape and keeps the
-    // fastest for every later call on that shape (tuned_choice).
-    bool narrow_ok = false, narrow = false;
+    int b_tile = 0, maxcj = 0, smem = 0, ntc = 64, nbs = 2, gq = 0, gslot = 0;
+    // K parts per tile of the contraction.  The tuner times the candidates on the first unscreened
+    // contraction of a shape and keeps the fastest for every later call on that shape.
     int kparts = T1_KPARTS;
     bool kparts_forced = false, tuned = false;
     std::string shape_key;
+    T1Args t1_args(const double *G, double *chi0R) const;
     void autotune(const double *G, double *chi0R, cudaStream_t st);
     void launch_t1(const T1Args &a, cudaStream_t st);
 };
@@ -986,7 +956,6 @@ struct TcChi0::Impl
 namespace {
 struct T1Choice
 {
-    bool narrow;
     int kparts;
     double ms;
 };
@@ -996,21 +965,7 @@ std::map<std::string, T1Choice> g_tuned;  // shape key -> choice (process-wide)
 
 namespace {
 using T1Fn = void (*)(T1Args, T1Maps);
-// The narrow producer layout serves the streamed (4-column-aligned, RA <= 16) cases with up
-// to 64 ABFs on atom J (its 96 registers a thread hold 64 accumulator columns, not 128).
-bool t1_narrow_ok(int ra, int ntc, bool sv) { return ra <= 16 && sv && ntc == 64; }
-
-int t1_threads(bool narrow) { return narrow ? T1Layout<true>::threads : T1Layout<false>::threads; }
-
-T1Fn t1_kernel(int ra, int ntc, bool sv, bool narrow)
-{
-    if (narrow) return ra == 13 ? k_t1_tc<13, 64, true, true> : k_t1_tc<16, 64, true, true>;
-    if (ra == 13 && sv) return ntc == 64 ? k_t1_tc<13, 64, true, false> : k_t1_tc<13, 128, true, false>;
-    if (ra == 13) return ntc == 64 ? k_t1_tc<13, 64, false, false> : k_t1_tc<13, 128, false, false>;
-    if (ra == 16 && sv) return ntc == 64 ? k_t1_tc<16, 64, true, false> : k_t1_tc<16, 128, true, false>;
-    if (ra == 16) return ntc == 64 ? k_t1_tc<16, 64, false, false> : k_t1_tc<16, 128, false, false>;
-    return ntc == 64 ? k_t1_tc<32, 64, false, false> : k_t1_tc<32, 128, false, false>;
-}
+T1Fn t1_kernel(int ntc) { return ntc == 48 ? k_t1_tc<48> : ntc == 64 ? k_t1_tc<64> : k_t1_tc<128>; }
 } // namespace
 
 TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st) : impl_(std::make_unique<Impl>())
@@ -1020,7 +975,9 @@ TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st)
     m.pr = pr;
     const long long nsup = g.n_sup;
     m.kpad = (nsup + 63) / 64 * 64;
-    m.nkc = static_cast<int>((nsup + CW - 1) / CW);
+    m.n4 = (g.n_ao + 3) / 4;
+    m.ng4 = g.n_c * m.n4;
+    m.nkc = (m.ng4 + 1) / 2;
     const char *env = std::getenv("LIBRPA_GB300_T1");
     m.t1_simt = env && std::string(env) == "simt";
     GB_REQUIRE(g.max_nao <= T1_MAXA, "the tensor-core chi0 kernel supports up to 32 NAOs per atom");
@@ -1052,6 +1009,19 @@ TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st)
         launch_d2f(C, m.Cf.get(), g.rows_c * nsup, st);
         m.Gf.alloc(2ull * g.n_c * g.n_ao * g.n_ao);
         return;
+    }
+    {
+        std::vector<long long> xo(g.n_at);
+        long long n = 0;
+        for (int I = 0; I < g.n_at; ++I)
+        {
+            xo[I] = n;
+            n += static_cast<long long>(m.ng4) * t1_rows(nao[I]) * nabf[I];
+        }
+        m.Xt.alloc(n);
+        m.xoff.alloc(xo.size());
+        m.xoff.upload(xo.data(), xo.size(), st);
+        GB_CUDA(cudaStreamSynchronize(st));  // xo goes out of scope
     }
     // T1 B operands grouped by species (same NAO and ABF counts) and their TMA maps
     std::vector<int> ajp(g.n_at), spec(g.n_at), spec_idx(g.n_at);
@@ -1088,7 +1058,7 @@ TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st)
             if (spec[J] != static_cast<int>(sp)) continue;
             const long long o = per_atom * spec_idx[J];
             k_cb_layout<<<static_cast<unsigned>(std::min<long long>((per_atom + 255) / 256, 152LL * 16)), 256, 0, st>>>(
-                C, g, J, ap, m.nkc, ktot, b.p[0] + o, b.p[1] + o, b.p[2] + o);
+                C, g, J, ap, m.n4, m.ng4, ktot, b.p[0] + o, b.p[1] + o, b.p[2] + o);
             GB_LAUNCH_CHECK();
         }
         const int NT = (nb + 15) / 16 * 16;
@@ -1096,8 +1066,6 @@ TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st)
             make_tmap_bf16(&m.maps.m[sp][p], b.p[p], ktot, nb, spec_count[sp], ktot, per_atom, 64, NT);
         m.maps.ktot[sp] = ktot;
     }
-    m.ajpad.alloc(ajp.size());
-    m.ajpad.upload(ajp.data(), ajp.size(), st);
     m.spec.alloc(spec.size());
     m.spec.upload(spec.data(), spec.size(), st);
     m.spec_idx.alloc(spec_idx.size());
@@ -1122,37 +1090,31 @@ TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st)
     }
     m.b_tile = (ntmax * 128 + 1023) / 1024 * 1024;
     m.maxcj = (T1_BM + minb - 1) / minb + 1;
-    m.ra = g.max_nao == 13 ? 13 : g.max_nao <= 16 ? 16 : 32;
-    m.ntc = ntmax <= 64 ? 64 : 128;
-    m.gj = 2 * JG;  // the streaming producers read 16 values of j per row i
-    for (int J = 0; J < g.n_at; ++J) m.gj = std::max(m.gj, ajp[J]);
-    // shared memory: A ring + at least two B stages + the G slots; fewer G slots than a tile of
-    // small row groups could touch only shortens such tiles
-    const int slot_bytes = 2 * rap(m.ra) * m.gj * 4;
-    const int base = T1_STAGES * NS * A_TILE + 1024 + 512;
+    m.ntc = ntmax <= 48 ? 48 : ntmax <= 64 ? 64 : 128;
+    // a G block of the largest atoms; 4 more floats keep the blocks of two groups on different banks
+    m.gq = 2 * g.max_nao;
+    m.gslot = m.gq * ((g.max_nao + JG - 1) / JG * JG) + 4;
+    // shared memory: at least two B stages + the G slots; fewer G slots than a tile of small row
+    // groups could touch only shortens such tiles
+    const int slot_bytes = (m.gslot + T1_CELLS) * 4;
+    const int base = 1024 + T1_XBYTES + 512;
     const int fit = (T1_SMEM_MAX - base - 2 * NS * m.b_tile) / slot_bytes;
     GB_REQUIRE(fit >= 1, "chi0 tile does not fit shared memory (too many ABFs or NAOs per atom)");
     m.maxcj = std::min(m.maxcj, fit);
     const int fixed = base + m.maxcj * slot_bytes;
     m.nbs = std::min(T1_MAXB, (T1_SMEM_MAX - fixed) / (NS * m.b_tile));
     m.smem = fixed + m.nbs * NS * m.b_tile;
-    const bool sv = g.n_ao % 4 == 0;
-    m.narrow_ok = t1_narrow_ok(m.ra, m.ntc, sv);
-    m.narrow = m.narrow_ok;
     // the cap, not this shape's own size: contractions of other shapes on other host threads share
     // the kernel, and a smaller value set by one of them would fail this one's launch
-    GB_CUDA(cudaFuncSetAttribute(t1_kernel(m.ra, m.ntc, sv, false), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 T1_SMEM_MAX));
-    if (m.narrow_ok)
-        GB_CUDA(cudaFuncSetAttribute(t1_kernel(m.ra, m.ntc, sv, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     T1_SMEM_MAX));
+    GB_CUDA(cudaFuncSetAttribute(t1_kernel(m.ntc), cudaFuncAttributeMaxDynamicSharedMemorySize, T1_SMEM_MAX));
     // the shape the tuner's choice is kept for: per-atom sizes, cells, pairs, SM count
     {
         std::string key = std::to_string(g.n_c) + ":" + std::to_string(g.n_ao) + ":" + std::to_string(pr.n_pairs) +
                           ":" + std::to_string(m.n_sm) + ":";
         for (int J = 0; J < g.n_at; ++J) key += std::to_string(nao[J]) + "/" + std::to_string(nabf[J]) + ",";
         m.shape_key = key;
-        // LIBRPA_GB300_T1_LAUNCH = "narrow:<kparts>" or "wide:<kparts>" fixes the choice (no tuning)
+        // LIBRPA_GB300_T1_LAUNCH = "wide:<kparts>" fixes the choice (no tuning); "narrow:" reads the same,
+        // there is one producer layout
         if (const char *fx = std::getenv("LIBRPA_GB300_T1_LAUNCH"))
         {
             const std::string v(fx);
@@ -1162,7 +1124,6 @@ TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st)
             const int kp = std::atoi(v.c_str() + c + 1);
             GB_REQUIRE((lay == "narrow" || lay == "wide") && kp >= 1 && kp <= T1_KPARTS_MAX,
                        "LIBRPA_GB300_T1_LAUNCH must read narrow:<kparts> or wide:<kparts>, kparts 1-8");
-            m.narrow = lay == "narrow" && m.narrow_ok;
             m.kparts = kp;
             m.kparts_forced = true;
             m.tuned = true;
@@ -1171,7 +1132,6 @@ TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st)
         auto it = m.tuned ? g_tuned.end() : g_tuned.find(key);
         if (it != g_tuned.end())
         {
-            m.narrow = it->second.narrow;
             m.kparts = it->second.kparts;
             m.kparts_forced = true;
             m.tuned = true;
@@ -1181,64 +1141,67 @@ TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st)
     GB_CUDA(cudaStreamSynchronize(st));
 }
 
-void TcChi0::Impl::launch_t1(const T1Args &a, cudaStream_t st)
-{
-    t1_kernel(ra, ntc, a.vec4 != 0, narrow)<<<n_work, t1_threads(narrow), smem, st>>>(a, maps);
-    GB_LAUNCH_CHECK();
-}
-
-// Times every candidate (producer layout x K parts per tile) on this contraction's own inputs,
-// one warm and one timed launch each, and keeps the fastest.  The candidates write chi0R; the
-// caller's own launch after the tuning overwrites it (zeroing it first when tiles are split).
-void TcChi0::Impl::autotune(const double *G, double *chi0R, cudaStream_t st)
+T1Args TcChi0::Impl::t1_args(const double *G, double *chi0R) const
 {
     T1Args a{};
     a.g = g;
     a.pr = pr;
-    a.X = X.get();
-    a.xsign = g.rows_c * g.n_sup;
+    a.Xt = Xt.get();
+    a.xoff = xoff.get();
     a.G = G;
     a.cadd = cadd.get();
     a.work = work.get();
     a.groups = groups.get();
     a.spec = spec.get();
     a.spec_idx = spec_idx.get();
-    a.aJpad = ajpad.get();
-    a.nkc = nkc;
+    a.n4 = n4;
+    a.ng4 = ng4;
     a.b_tile = b_tile;
     a.nbs = nbs;
-    a.gj = gj;
+    a.gq = gq;
+    a.gslot = gslot;
     a.maxcj = maxcj;
-    a.vec4 = g.n_ao % 4 == 0 ? 1 : 0;
     a.out = chi0R;
     a.err = err.get();
+    return a;
+}
+
+void TcChi0::Impl::launch_t1(const T1Args &a, cudaStream_t st)
+{
+    t1_kernel(ntc)<<<n_work, T1_THREADS, smem, st>>>(a, maps);
+    GB_LAUNCH_CHECK();
+}
+
+// Times every candidate count of K parts per tile on this contraction's own inputs, one warm and
+// one timed launch each, and keeps the fastest.  The candidates write chi0R; the caller's own launch
+// after the tuning overwrites it (zeroing it first when tiles are split).
+void TcChi0::Impl::autotune(const double *G, double *chi0R, cudaStream_t st)
+{
+    const T1Args a = t1_args(G, chi0R);
     cudaEvent_t e0, e1;
     GB_CUDA(cudaEventCreate(&e0));
     GB_CUDA(cudaEventCreate(&e1));
-    T1Choice best{narrow, kparts, 1e30};
+    T1Choice best{kparts, 1e30};
     const int kp_cand[] = {1, 2, 4, 8};
-    for (int lay = 0; lay < (narrow_ok ? 2 : 1); ++lay)
-        for (int kp : kp_cand)
-        {
-            if (kp > T1_KPARTS_MAX || (kp > 1 && nkc < 2 * kp)) continue;
-            narrow = lay == 0 && narrow_ok;
-            kparts = kp;
-            kparts_forced = true;
-            all_active = false;
-            build_work(nullptr, st);
-            if (n_work == 0) continue;
-            launch_t1(a, st);
-            GB_CUDA(cudaEventRecord(e0, st));
-            launch_t1(a, st);
-            GB_CUDA(cudaEventRecord(e1, st));
-            GB_CUDA(cudaEventSynchronize(e1));
-            float ms = 0.0f;
-            GB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            if (ms < best.ms) best = T1Choice{narrow, kp, ms};
-        }
+    for (int kp : kp_cand)
+    {
+        if (kp > T1_KPARTS_MAX || (kp > 1 && nkc < 2 * kp)) continue;
+        kparts = kp;
+        kparts_forced = true;
+        all_active = false;
+        build_work(nullptr, st);
+        if (n_work == 0) continue;
+        launch_t1(a, st);
+        GB_CUDA(cudaEventRecord(e0, st));
+        launch_t1(a, st);
+        GB_CUDA(cudaEventRecord(e1, st));
+        GB_CUDA(cudaEventSynchronize(e1));
+        float ms = 0.0f;
+        GB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        if (ms < best.ms) best = T1Choice{kp, ms};
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    narrow = best.narrow;
     kparts = best.kparts;
     kparts_forced = true;
     all_active = false;
@@ -1323,7 +1286,7 @@ TcChi0::~TcChi0() = default;
 
 void TcChi0::launch_choice(int &narrow, int &kparts) const
 {
-    narrow = impl_->narrow ? 1 : 0;
+    narrow = 0;  // one producer layout
     kparts = impl_->kparts;
 }
 
@@ -1345,7 +1308,12 @@ int TcChi0::prepare(const double *G, cudaStream_t st)
     tc_gemm_split(m.csplit.mat(g.rows_c, m.kpad, 0), m.gs.mat(nsup, m.kpad, nsup * m.kpad), static_cast<int>(g.rows_c),
                   static_cast<int>(nsup), static_cast<int>(nsup), 2, m.X.get(), nsup, g.rows_c * nsup, false,
                   m.err.get(), st);
-    return 2;
+    if (m.t1_simt) return 2;
+    const int mu_tiles = (g.max_nabf + 31) / 32;
+    k_x_layout<<<dim3((m.ng4 + 7) / 8, g.n_at * mu_tiles, t1_rows(g.max_nao) / T1_XD), 256, 0, st>>>(m.X.get(), g.rows_c * nsup, g, m.n4, m.ng4,
+                                                                         mu_tiles, m.xoff.get(), m.Xt.get());
+    GB_LAUNCH_CHECK();
+    return 3;
 }
 
 int TcChi0::contract(const double *G, double *chi0R, const unsigned char *active, bool zero_first, cudaStream_t st)
@@ -1370,31 +1338,13 @@ int TcChi0::contract(const double *G, double *chi0R, const unsigned char *active
     }
     else
     {
-        T1Args a;
-        a.g = g;
-        a.pr = m.pr;
-        a.X = m.X.get();
-        a.xsign = g.rows_c * nsup;
-        a.G = G;
-        a.cadd = m.cadd.get();
-        a.work = m.work.get();
-        a.groups = m.groups.get();
-        a.spec = m.spec.get();
-        a.spec_idx = m.spec_idx.get();
-        a.aJpad = m.ajpad.get();
-        a.nkc = m.nkc;
-        a.b_tile = m.b_tile;
-        a.nbs = m.nbs;
-        a.gj = m.gj;
-        a.maxcj = m.maxcj;
-        a.vec4 = g.n_ao % 4 == 0 ? 1 : 0;
-        a.out = chi0R;
-        a.err = m.err.get();
+        const T1Args a = m.t1_args(G, chi0R);
         if (m.n_work > 0)
         {
             m.launch_t1(a, st);
-            k_t2<<<dim3(m.n_groups, T2_TILES * T2_TILES), T2_THREADS, 0, st>>>(m.X.get(), g.rows_c * nsup, g, m.pr,
-                                                                             m.groups.get(), chi0R);
+            const int tiles = (g.max_nabf + T2_TILE - 1) / T2_TILE;
+            k_t2<<<dim3(m.n_groups, tiles * tiles), T2_THREADS, 0, st>>>(m.Xt.get(), m.xoff.get(), m.n4, g, m.pr,
+                                                                       m.groups.get(), tiles, chi0R);
             GB_LAUNCH_CHECK();
             launches += 2;
         }

@@ -83,6 +83,30 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity)
     return false;
 }
 
+// The same for a wait that is long beside the work of the other warps on its scheduler: it sleeps NAP
+// nanoseconds between polls, and is bounded by the number of polls alone (reading %globaltimer costs
+// more than a short wait).
+template <uint32_t NAP>
+__device__ __forceinline__ bool mbar_wait_nap(uint64_t *bar, uint32_t parity)
+{
+    constexpr uint32_t kPolls = 1u << 24;
+    for (uint32_t i = 0; i < kPolls; ++i)
+    {
+        if (mbar_try_wait(bar, parity)) return true;
+        if (NAP > 0) __nanosleep(NAP);
+    }
+    return false;
+}
+
+// One lane of a converged warp.  Code that a whole warp runs with this around the issuing instructions
+// keeps their operands in uniform registers; under `lane == 0` each operand is moved there first.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ void fence_proxy_async_smem()
 {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
