@@ -224,10 +224,10 @@ __device__ __forceinline__ void t1_row(uint32_t xs, uint32_t ga, uint32_t gb, fl
 // Bounds: 128 FP32 FMAs per clock per SM (the rows loop alone reaches 92), next to it the shared-memory
 // path: a G value loaded serves the thread's 8 columns, an X value its j.  The two warpgroups work on
 // alternate chunks, so that the split and the hand-over of one run under the FMAs of the other.
-// Measured (13 NAO / 40 ABF atoms, per tau): 128 atoms at Gamma 21.2 -> 13.6 ms, 8 -> 12 mixed-species
-// atoms a tile (5/20, 13/60, 26/110; 48 atoms) 20.0 -> 4.0 ms, against two threads a row that wrote E to
-// shared memory with one drain warp issuing everything.  What is left: the producers' two warps per
-// scheduler, 48 of 128 FMAs per clock over the whole kernel.
+// Measured on one GB300 against two threads a row that wrote E to shared memory, with one drain warp
+// issuing everything, the whole chi0 stage: 128 atoms of 13/40 at Gamma 426 -> 289 ms, 48 atoms of 5/20,
+// 13/60 and 26/110 528 -> 112 ms, 16 atoms of 13/40 on 3x3x3 k 578 -> 394 ms.  What is left: two producer
+// warps per scheduler, 48 of 128 FMAs per clock over the kernel.
 template <int NJ, typename Fetch>
 __device__ __forceinline__ bool t1_unit(uint32_t xring, int &slot, const Fetch &fetch, uint32_t gs,
                                         int gq, int nq, int nhalf, uint32_t atile, uint64_t *full, uint64_t *empty, uint32_t &use,
