@@ -94,55 +94,85 @@ __global__ void __launch_bounds__(256) k_chol_diag(T *__restrict__ Aall, int N, 
     for (int i = threadIdx.x; i < nb; i += blockDim.x) diag[static_cast<long long>(b) * N + k0 + i] = cre(D[i][i]);
 }
 
-// Real diagonal block for the tensor-core panel solve: factor L11 as k_chol_diag does and also
-// form W = L11^-1 (lower triangular, FP64) into Wb[b][64][64], so that the panel becomes the
-// product L21 = A21 W^T.  Thread c (< nb) builds column c of W by forward substitution,
-// W_cc = 1 / L_cc, W_ic = -(sum_{k=c}^{i-1} L_ik W_kc) / L_ii.  Dynamic shared memory: D, W.
-constexpr int DINV_SMEM = 2 * OZAKI_NB * (OZAKI_NB + 1) * static_cast<int>(sizeof(double));
-__global__ void __launch_bounds__(256) k_chol_diag_inv(double *__restrict__ Aall, int N, int k0,
-                                                      double *__restrict__ diag, int *__restrict__ bad,
-                                                      double *__restrict__ Wb)
+// Real diagonal block of the tensor-core Cholesky: factor the nb x nb block at k0 in place, record the
+// diagonal of L, and with INV form W = L11^-1 (lower triangular, FP64) into Wb[b][64][64], so that the
+// panel becomes the product L21 = A21 W^T.
+//
+// Right-looking, the block in registers: thread 4 i + s holds the columns 4 k + s of row i.  Step p
+// scales column p, and with INV row p of what has been made of the identity, then subtracts their outer
+// product from the rows below; a row's columns up to p belong to the inverse and the later ones to A, so
+// one array of 16 holds both.  Bound by the pivots' chain and the FP64 pipe (1.6 FMAs per clock per SM):
+// the pivot takes one reciprocal square root instead of a square root and a division, two dependent
+// sequences of several hundred clocks each.  One GB300, a 64 x 64 block with its inverse: 216 -> 128 us.
+template <bool INV>
+__global__ void __launch_bounds__(256) k_chol_diag64(double *__restrict__ Aall, int N, int k0, double *__restrict__ diag,
+                                                    int *__restrict__ bad, double *__restrict__ Wb)
 {
     constexpr int NBT = OZAKI_NB;
-    extern __shared__ double dsm[];
-    double (*D)[NBT + 1] = reinterpret_cast<double (*)[NBT + 1]>(dsm);
-    double (*W)[NBT + 1] = reinterpret_cast<double (*)[NBT + 1]>(dsm + NBT * (NBT + 1));
-    const int b = blockIdx.x;
-    double *A = Aall + static_cast<long long>(b) * N * N;
-    const int nb = min(NBT, N - k0);
-    factor_diag<double, NBT>(A, N, k0, nb, D, bad + b);
-    for (int t = threadIdx.x; t < nb * nb; t += blockDim.x)
-    {
-        const int i = t / nb, j = t % nb;
-        if (j <= i) A[static_cast<long long>(k0 + i) * N + k0 + j] = D[i][j];
-    }
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) diag[static_cast<long long>(b) * N + k0 + i] = D[i][i];
-    __shared__ double invd[NBT];
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) invd[i] = 1.0 / D[i][i];
-    __syncthreads();
-    const int c = threadIdx.x;
-    if (c < nb)
-    {
-        W[c][c] = invd[c];
-        for (int i = c + 1; i < nb; ++i)
+    static_assert(NBT == 64, "four threads a row, 16 columns each");
+    __shared__ double col[NBT], U[NBT], sinv;
+    const int b = blockIdx.x, nb = min(NBT, N - k0);
+    const int i = static_cast<int>(threadIdx.x) / 4, s = threadIdx.x % 4;
+    double *row = Aall + static_cast<long long>(b) * N * N + static_cast<long long>(k0 + i) * N + k0;
+    double v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = i < nb && 4 * k + s <= i ? row[4 * k + s] : 0.0;
+#pragma unroll
+    for (int kp = 0; kp < 16; ++kp)
+#pragma unroll 1
+        for (int sp = 0; sp < 4; ++sp)
         {
-            double s0 = 0.0, s1 = 0.0;  // two chains for the dependent FMA latency
-            int k = c;
-            for (; k + 1 < i; k += 2)
+            const int p = 4 * kp + sp;
+            if (p >= nb) break;
+            if (i == p && s == sp)
             {
-                s0 = fma(D[i][k], W[k][c], s0);
-                s1 = fma(D[i][k + 1], W[k + 1][c], s1);
+                const double d = fmax(v[kp], 1e-300);
+                if (!(v[kp] > 0.0)) bad[b] = 1;
+                const double inv = rsqrt(d);
+                sinv = inv;
+                double l = d * inv;  // sqrt(d), corrected to its own rounding
+                l = fma(fma(-l, l, d), 0.5 * inv, l);
+                row[p] = l;
+                diag[static_cast<long long>(b) * N + k0 + p] = l;
             }
-            if (k < i) s0 = fma(D[i][k], W[k][c], s0);
-            W[i][c] = -(s0 + s1) * invd[i];
+            __syncthreads();
+            const double inv = sinv;
+            if (i > p && i < nb && s == sp)
+            {
+                const double c = v[kp] * inv;
+                row[p] = c;
+                col[i] = c;
+                U[i] = c;
+                v[kp] = 0.0;
+            }
+            if (INV && i == p)
+            {
+#pragma unroll
+                for (int k = 0; k <= kp; ++k)
+                {
+                    const int j = 4 * k + s;
+                    if (j < p) v[k] *= inv;
+                    if (j == p) v[k] = inv;
+                    if (j <= p) U[j] = v[k];
+                }
+            }
+            __syncthreads();
+            if (i > p && i < nb)
+            {
+                const double c = col[i];
+#pragma unroll
+                for (int k = INV ? 0 : kp; k < 16; ++k)
+                {
+                    const int j = 4 * k + s;
+                    if (j <= i && (INV || j > p)) v[k] = fma(-c, U[j], v[k]);
+                }
+            }
         }
-    }
-    __syncthreads();
-    double *Wo = Wb + static_cast<long long>(b) * NBT * NBT;
-    for (int t = threadIdx.x; t < NBT * NBT; t += blockDim.x)
+    if constexpr (INV)
     {
-        const int i = t / NBT, j = t % NBT;
-        Wo[t] = (i < nb && j <= i) ? W[i][j] : 0.0;
+        double *w = Wb + (static_cast<long long>(b) * NBT + i) * NBT;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) w[4 * k + s] = i < nb && 4 * k + s <= i ? v[k] : 0.0;
     }
 }
 
@@ -310,10 +340,6 @@ int chol_batched_r(double *A, int N, int batch, double *diag, int *bad, cudaStre
 int chol_batched_r_ozaki(double *A, int N, int batch, double *diag, int *bad, OzakiWork &w, cudaStream_t st)
 {
     constexpr int NBO = OZAKI_NB;
-    static PerDeviceOnce attr;
-    attr.run([] {
-        GB_CUDA(cudaFuncSetAttribute(k_chol_diag_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, DINV_SMEM));
-    });
     int launches = 0;
     for (int k0 = 0; k0 < N; k0 += NBO)
     {
@@ -321,13 +347,13 @@ int chol_batched_r_ozaki(double *A, int N, int batch, double *diag, int *bad, Oz
         const int rows_below = N - k0 - nb;
         if (rows_below == 0)
         {
-            k_chol_diag<double, NBO><<<batch, 256, 0, st>>>(A, N, k0, diag, bad);
+            k_chol_diag64<false><<<batch, 256, 0, st>>>(A, N, k0, diag, bad, nullptr);
             GB_LAUNCH_CHECK();
             ++launches;
             continue;
         }
         // every panel with rows below it is a full 64-wide one (panels step by 64)
-        k_chol_diag_inv<<<batch, 256, DINV_SMEM, st>>>(A, N, k0, diag, bad, w.winv);
+        k_chol_diag64<true><<<batch, 256, 0, st>>>(A, N, k0, diag, bad, w.winv);
         GB_LAUNCH_CHECK();
         launches += 1 + ozaki_panel_solve(A, N, batch, k0, w, st);
         launches += ozaki_trailing_update(A, N, batch, k0 + nb, k0, nb, w, st);

@@ -1,5 +1,5 @@
 // Panel solve and trailing update of the real batched Cholesky on the tensor cores, to FP64
-// accuracy.  The panel L21 = A21 W^T (W = L11^-1 from k_chol_diag_inv) and the update below are
+// accuracy.  The panel L21 = A21 W^T (W = L11^-1 from k_chol_diag64) and the update below are
 // the same exact slice products; they differ only in the operands and in the epilogue, which
 // writes the panel and subtracts from the trailing matrix (k_ozaki_syrk<TRSM>).
 //
