@@ -22,6 +22,8 @@
 // ([(a,p), s]), Yw = W Y ([b, (p,s)]) and H = Yw U over (b, s).  The dense U holds N_abf n_ao^2 values, which bounds
 // this formulation to cells of a few hundred orbitals; larger cells need the atom-pair-sparse
 // form of the χ0 contraction.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -72,83 +74,131 @@ __global__ void k_one_minus(double *__restrict__ A, int N, int batch)
     }
 }
 
-// Solve A X = B in place (B <- X) by Gauss-Jordan elimination with partial pivoting, one CTA per
-// batch entry: A N x N, B N x M, both row-major in global memory.  *bad is set when a pivot is 0.
-__global__ void __launch_bounds__(256) k_gj_solve(double *__restrict__ Aall, double *__restrict__ Ball, int N, int M,
-                                                  int *__restrict__ bad)
+// Solve A X = B in place (B <- X) by Gauss-Jordan elimination with partial pivoting: A N x N, B N x M,
+// both row-major in global memory, A destroyed.  *bad is set when a pivot is 0.
+//
+// A cluster of GJ_CL CTAs per batch entry shares the columns of [A | B], 4 adjacent ones at a time in
+// turn, so that a CTA reads and writes its own columns only.  The owner of column k searches it for the
+// pivot and hands pivot and column to the others through distributed shared memory; then each CTA swaps,
+// scales and eliminates in its columns right of k.  Bound by the FP64 pipe of the CTAs (1.6 FMAs per clock
+// per SM) and, below N ~ 100, by the step's two hand-overs; with one CTA per entry, 16 of 152 SMs worked,
+// 3.80 ms for 16 entries of N = M = 102 (now 0.97).
+constexpr int GJ_CL = 8;
+
+__global__ void __cluster_dims__(GJ_CL, 1, 1) __launch_bounds__(256)
+    k_gj_solve(double *__restrict__ Aall, double *__restrict__ Ball, int N, int M, int *__restrict__ bad)
 {
-    double *A = Aall + static_cast<size_t>(blockIdx.x) * N * N;
-    double *B = Ball + static_cast<size_t>(blockIdx.x) * N * M;
-    extern __shared__ double col[];  // column k of A before the elimination step
-    __shared__ double rv[256];
-    __shared__ int ri[256];
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const int r = static_cast<int>(cl.block_rank()), m = static_cast<int>(blockIdx.x) / GJ_CL;
+    double *A = Aall + static_cast<size_t>(m) * N * N;
+    double *B = Ball + static_cast<size_t>(m) * N * M;
+    extern __shared__ double sm[];
+    double *col = sm;          // [2][N]: column k before the elimination step, rows k and pivot swapped
+    double *rowk = sm + 2 * N; // row k of this CTA's columns
+    __shared__ double rv[8];
+    __shared__ int ri[8], piv_of[2];
+    // local column jl is column j of [A | B], in ascending order
+    const int groups = (N + M + 3) / 4, mine = groups > r ? (groups - r + GJ_CL - 1) / GJ_CL : 0;
+    int nl = 4 * mine;
+    if (mine > 0 && (groups - 1) % GJ_CL == r) nl -= 4 * groups - (N + M);
+    auto column = [&](int jl) { return ((jl / 4) * GJ_CL + r) * 4 + jl % 4; };
+    auto at = [&](int i, int j) -> double * {
+        return j < N ? A + static_cast<size_t>(i) * N + j : B + static_cast<size_t>(i) * M + (j - N);
+    };
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     for (int k = 0; k < N; ++k)
     {
-        // pivot: largest |A[i][k]|, i >= k
-        double best = -1.0;
-        int bi = k;
-        for (int i = k + threadIdx.x; i < N; i += blockDim.x)
+        const int buf = k & 1;
+        if ((k / 4) % GJ_CL == r)
         {
-            const double v = fabs(A[static_cast<size_t>(i) * N + k]);
-            if (v > best)
+            // pivot: largest |A[i][k]|, i >= k, the first of equals
+            double best = -1.0;
+            int bi = k;
+            for (int i = k + threadIdx.x; i < N; i += 256)
             {
-                best = v;
-                bi = i;
+                const double v = fabs(*at(i, k));
+                if (v > best)
+                {
+                    best = v;
+                    bi = i;
+                }
             }
-        }
-        rv[threadIdx.x] = best;
-        ri[threadIdx.x] = bi;
-        __syncthreads();
-        for (int s = blockDim.x / 2; s > 0; s >>= 1)
-        {
-            if (threadIdx.x < s && (rv[threadIdx.x + s] > rv[threadIdx.x] ||
-                                    (rv[threadIdx.x + s] == rv[threadIdx.x] && ri[threadIdx.x + s] < ri[threadIdx.x])))
+            for (int o = 16; o > 0; o >>= 1)
             {
-                rv[threadIdx.x] = rv[threadIdx.x + s];
-                ri[threadIdx.x] = ri[threadIdx.x + s];
+                const double v = __shfl_xor_sync(0xffffffffu, best, o);
+                const int vi = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (v > best || (v == best && vi < bi))
+                {
+                    best = v;
+                    bi = vi;
+                }
+            }
+            if (lane == 0)
+            {
+                rv[warp] = best;
+                ri[warp] = bi;
             }
             __syncthreads();
-        }
-        const int piv = ri[0];
-        if (threadIdx.x == 0 && !(rv[0] > 0.0)) atomicExch(bad, 1);
-        __syncthreads();
-        if (piv != k)
-        {
-            for (int j = threadIdx.x; j < N; j += blockDim.x)
+            best = rv[0];
+            bi = ri[0];
+            for (int q = 1; q < 8; ++q)
+                if (rv[q] > best || (rv[q] == best && ri[q] < bi))
+                {
+                    best = rv[q];
+                    bi = ri[q];
+                }
+            if (threadIdx.x == 0 && !(best > 0.0)) atomicExch(bad, 1);
+            for (int t = threadIdx.x; t < N * GJ_CL; t += 256)
             {
-                const double t = A[static_cast<size_t>(k) * N + j];
-                A[static_cast<size_t>(k) * N + j] = A[static_cast<size_t>(piv) * N + j];
-                A[static_cast<size_t>(piv) * N + j] = t;
+                const int q = t / N, i = t % N;
+                cl.map_shared_rank(col, q)[buf * N + i] = *at(i == k ? bi : i == bi ? k : i, k);
             }
-            for (int j = threadIdx.x; j < M; j += blockDim.x)
-            {
-                const double t = B[static_cast<size_t>(k) * M + j];
-                B[static_cast<size_t>(k) * M + j] = B[static_cast<size_t>(piv) * M + j];
-                B[static_cast<size_t>(piv) * M + j] = t;
-            }
+            if (threadIdx.x < GJ_CL) cl.map_shared_rank(piv_of, threadIdx.x)[buf] = bi;
         }
-        __syncthreads();
-        const double pv = A[static_cast<size_t>(k) * N + k];
+        cl.sync();
+        const double *ck = col + buf * N;
+        const int piv = piv_of[buf];
+        const double pv = ck[k];
         const double inv = pv != 0.0 ? 1.0 / pv : 0.0;
-        __syncthreads();
-        for (int j = threadIdx.x; j < N; j += blockDim.x) A[static_cast<size_t>(k) * N + j] *= inv;
-        for (int j = threadIdx.x; j < M; j += blockDim.x) B[static_cast<size_t>(k) * M + j] *= inv;
-        for (int i = threadIdx.x; i < N; i += blockDim.x) col[i] = A[static_cast<size_t>(i) * N + k];
-        __syncthreads();
-        // eliminate column k from every other row
-        for (long long t = threadIdx.x; t < static_cast<long long>(N) * (N + M); t += blockDim.x)
+        // this CTA's columns right of k
+        const int gk = k / 4;
+        const int jl0 = (gk > r ? (gk - r + GJ_CL - 1) / GJ_CL * 4 : 0) + (gk % GJ_CL == r ? k % 4 + 1 : 0);
+        for (int jl = jl0 + threadIdx.x; jl < nl; jl += 256)
         {
-            const int i = static_cast<int>(t / (N + M)), j = static_cast<int>(t % (N + M));
-            if (i == k) continue;
-            const double f = col[i];
-            if (f == 0.0) continue;
-            if (j < N)
-                A[static_cast<size_t>(i) * N + j] -= f * A[static_cast<size_t>(k) * N + j];
-            else
-                B[static_cast<size_t>(i) * M + (j - N)] -= f * B[static_cast<size_t>(k) * M + (j - N)];
+            const int j = column(jl);
+            double x = *at(k, j);
+            if (piv != k)
+            {
+                const double y = *at(piv, j);
+                *at(piv, j) = x;
+                x = y;
+            }
+            x *= inv;
+            *at(k, j) = x;
+            rowk[jl] = x;
+        }
+        __syncthreads();
+        const int na = nl - jl0;
+        for (long long t = threadIdx.x; t < static_cast<long long>(N) * na; t += 256)
+        {
+            const int i = static_cast<int>(t / na), jl = jl0 + static_cast<int>(t % na);
+            const double f = ck[i];
+            if (i == k || f == 0.0) continue;
+            *at(i, column(jl)) -= f * rowk[jl];
         }
         __syncthreads();
     }
+    cl.sync();  // no CTA leaves while another may still write into it
+}
+
+size_t gj_smem(int N, int M) { return sizeof(double) * (2 * static_cast<size_t>(N) + (N + M) / GJ_CL + 8); }
+
+void launch_gj_solve(double *A, double *B, int N, int M, int batch, int *bad, cudaStream_t st)
+{
+    static PerDeviceOnce attr;
+    attr.run([] { GB_CUDA(cudaFuncSetAttribute(k_gj_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); });
+    k_gj_solve<<<batch * GJ_CL, 256, gj_smem(N, M), st>>>(A, B, N, M, bad);
+    GB_LAUNCH_CHECK();
 }
 
 // Sig[w][pq] += c[w] (S+ + S-)/2 + i sn[w] (S+ - S-)/2
@@ -1157,10 +1207,8 @@ void build_g0w0_gamma(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
         GB_CUDA(cudaMemcpyAsync(Y.get() + w * NN, Sc.get(), sizeof(double) * NN, cudaMemcpyDeviceToDevice, st));
     DevBuf<int> bad(1);
     bad.zero(st);
-    const size_t gj_smem = sizeof(double) * N;
-    GB_REQUIRE(gj_smem <= 48 * 1024, "auxiliary basis too large for the Gamma-point W_c solve");
-    k_gj_solve<<<nw, 256, gj_smem, st>>>(X.get(), Y.get(), N, N, bad.get());
-    GB_LAUNCH_CHECK();
+    GB_REQUIRE(N <= 6144, "auxiliary basis too large for the Gamma-point W_c solve");
+    launch_gj_solve(X.get(), Y.get(), N, N, nw, bad.get(), st);
     launch_dgemm(N, N, N, Sc.get(), N, 0, Y.get(), N, NN, Wf.get(), N, NN, nw, 1.0, 0.0, st);
     {
         // W_c(omega) -= S_c S_c for every frequency: one GEMM with a column of -1
@@ -1396,8 +1444,7 @@ void build_g0w0_kgrid(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
                 }
             return E;
         };
-        const size_t gj_smem = sizeof(double) * N2w;
-        GB_REQUIRE(gj_smem <= 48 * 1024, "auxiliary basis too large for the W_c solve");
+        GB_REQUIRE(N2w <= 6144, "auxiliary basis too large for the W_c solve");
         for (int q = 0; q < nq; ++q)
         {
             const int kq = pt.ibz_rep[q];
@@ -1520,8 +1567,7 @@ void build_g0w0_kgrid(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
             GB_LAUNCH_CHECK();
             for (int w = 0; w < nw; ++w)
                 GB_CUDA(cudaMemcpyAsync(Ye.get() + w * M4w, Sce.get(), sizeof(double) * M4w, cudaMemcpyDeviceToDevice, st));
-            k_gj_solve<<<nw, 256, gj_smem, st>>>(Xe.get(), Ye.get(), N2w, N2w, bad.get());
-            GB_LAUNCH_CHECK();
+            launch_gj_solve(Xe.get(), Ye.get(), N2w, N2w, nw, bad.get(), st);
             launch_dgemm(N2w, N2w, N2w, Sce.get(), N2w, 0, Ye.get(), N2w, M4w, We.get(), N2w, M4w, nw, 1.0, 0.0, st);
             launch_dgemm(nw, static_cast<int>(M4w), 1, d_ones.get(), 1, 0, ScSc.get(), M4w, 0, We.get(), M4w, 0, 1, 1.0, 1.0, st);
             const double *Wout = We.get();
