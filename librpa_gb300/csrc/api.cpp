@@ -305,6 +305,7 @@ void librpa_finalize_global(void)
     std::lock_guard<std::mutex> lk(g_mu);
     for (auto &p : g_instances)
         if (p) gb::release_kept(*p);
+    gb::release_idle_arenas();
 }
 
 void librpa_print_profile(void)
@@ -419,6 +420,8 @@ void librpa_destroy_handler(LibrpaHandler *h)
         {
             gb::release_kept(*g_instances[id]);
             g_instances[id].reset();
+            if (std::none_of(g_instances.begin(), g_instances.end(), [](const auto &p) { return static_cast<bool>(p); }))
+                gb::release_idle_arenas();
         }
     }
     delete h;

@@ -4,6 +4,10 @@
 #include <cuComplex.h>
 #include <cuda_runtime.h>
 
+#include <vector>
+
+#include "common.h"
+
 namespace gb {
 
 // In-place lower Cholesky of batch row-major N x N matrices (Hermitian / symmetric, lower
@@ -27,9 +31,9 @@ struct OzakiWork
     void *wslices = nullptr;   // [batch][slice][2 OZAKI_NB][OZAKI_NB] bf16: its rows (upper half zero)
     int *wexpo = nullptr;      // [batch][2 OZAKI_NB]
     int *err = nullptr;
+    std::vector<DevBuf<unsigned char>> own;  // what the pointers above point into
 };
-void ozaki_alloc(OzakiWork &w, int N, int batch);
-void ozaki_free(OzakiWork &w);
+void ozaki_alloc(OzakiWork &w, int N, int batch, cudaStream_t st);
 int chol_batched_r_ozaki(double *A, int N, int batch, double *diag, int *bad, OzakiWork &w, cudaStream_t st);
 // A[s0:, s0:] (lower) -= L21 L21^T with L21 = A[s0:, k0:k0+nb]; returns launches
 int ozaki_trailing_update(double *A, int N, int batch, int s0, int k0, int nb, OzakiWork &w, cudaStream_t st);

@@ -45,7 +45,43 @@ struct Error : std::runtime_error
 // kernel surfaces at the next synchronising call, which GB_CUDA also checks.
 #define GB_LAUNCH_CHECK() GB_CUDA(cudaGetLastError())
 
-// Owning device allocation (cudaMalloc / cudaFree), move-only.
+// Device memory kept between calls (device_arena.cpp).  While an ArenaScope is open on a thread, the
+// DevBufs it makes take their memory from the scope's arena: all GPU work on them must be on the scope's
+// stream, and they must be gone when the scope ends.  ArenaPause: DevBufs that outlive the call.
+class DeviceArena;
+DeviceArena *current_arena();
+void *arena_take(DeviceArena *a, size_t bytes);
+void arena_give(DeviceArena *a, void *p);
+void release_idle_arenas();
+// cudaMalloc; where it fails, once more after what the arenas hold idle has gone back to the driver
+void *device_malloc(size_t bytes);
+
+class ArenaScope
+{
+public:
+    explicit ArenaScope(cudaStream_t st);
+    ~ArenaScope();
+    ArenaScope(const ArenaScope &) = delete;
+    ArenaScope &operator=(const ArenaScope &) = delete;
+
+private:
+    cudaStream_t st_;
+    DeviceArena *prev_;
+};
+
+class ArenaPause
+{
+public:
+    ArenaPause();
+    ~ArenaPause();
+    ArenaPause(const ArenaPause &) = delete;
+    ArenaPause &operator=(const ArenaPause &) = delete;
+
+private:
+    DeviceArena *prev_;
+};
+
+// Owning device allocation (the thread's arena, or cudaMalloc / cudaFree), move-only.
 template <typename T>
 class DevBuf
 {
@@ -55,13 +91,13 @@ public:
     ~DevBuf() { release(); }
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p_(o.p_), n_(o.n_) { o.p_ = nullptr; o.n_ = 0; }
+    DevBuf(DevBuf &&o) noexcept : p_(o.p_), n_(o.n_), arena_(o.arena_) { o.p_ = nullptr; o.n_ = 0; }
     DevBuf &operator=(DevBuf &&o) noexcept
     {
         if (this != &o)
         {
             release();
-            p_ = o.p_; n_ = o.n_;
+            p_ = o.p_; n_ = o.n_; arena_ = o.arena_;
             o.p_ = nullptr; o.n_ = 0;
         }
         return *this;
@@ -70,12 +106,16 @@ public:
     {
         release();
         if (n == 0) return;
-        GB_CUDA(cudaMalloc(&p_, n * sizeof(T)));
+        arena_ = current_arena();
+        p_ = static_cast<T *>(arena_ ? arena_take(arena_, n * sizeof(T)) : device_malloc(n * sizeof(T)));
         n_ = n;
     }
     void release()
     {
-        if (p_) cudaFree(p_);
+        if (p_ && arena_)
+            arena_give(arena_, p_);
+        else if (p_)
+            cudaFree(p_);
         p_ = nullptr;
         n_ = 0;
     }
@@ -100,6 +140,7 @@ public:
 private:
     T *p_ = nullptr;
     size_t n_ = 0;
+    DeviceArena *arena_ = nullptr;
 };
 
 // A device copy of a host vector, staged on stream st.

@@ -298,10 +298,9 @@ struct EcChol::Impl
     // complex M' is factored as its real 2N x 2N embedding (emb) by the same kernels
     bool ozaki = false, emb = false;
     OzakiWork oz;
-    ~Impl() { ozaki_free(oz); }
 };
 
-EcChol::EcChol(int N, int nw, bool complex_path, int qb, bool fp64_products) : impl_(std::make_unique<Impl>())
+EcChol::EcChol(int N, int nw, bool complex_path, int qb, bool fp64_products, cudaStream_t st) : impl_(std::make_unique<Impl>())
 {
     Impl &m = *impl_;
     m.N = N;
@@ -330,8 +329,8 @@ EcChol::EcChol(int N, int nw, bool complex_path, int qb, bool fp64_products) : i
         m.Mpr.alloc(nmat * N * N);
     // V (one per q) and, for real matrices, M' go through the tensor-core Cholesky
     m.ozaki = !complex_path && !fp64_products && N > OZAKI_NB;
-    if (m.ozaki) ozaki_alloc(m.oz, N, static_cast<int>(nmat));
-    if (m.emb) ozaki_alloc(m.oz, 2 * N, static_cast<int>(nmat));
+    if (m.ozaki) ozaki_alloc(m.oz, N, static_cast<int>(nmat), st);
+    if (m.emb) ozaki_alloc(m.oz, 2 * N, static_cast<int>(nmat), st);
     if (fp64_products)
     {
         const size_t nn = static_cast<size_t>(N) * N;

@@ -16,7 +16,7 @@ public:
     // otherwise Gamma-only real parts; qb: q points whose M' = I - L^H chi0 L are factorised
     // in one batch; fp64_products: M = L^H chi0 L by FP64 CUDA-core GEMMs instead of the
     // split-precision tensor-core GEMMs.
-    EcChol(int N, int nw, bool complex_path, int qb, bool fp64_products = false);
+    EcChol(int N, int nw, bool complex_path, int qb, bool fp64_products, cudaStream_t st);
     ~EcChol();
     // V = L L^H in place for nb (<= qb) Coulomb matrices stored one after another (N x N each).
     // bad[b] != 0 where V has no Cholesky factor (not positive definite: the Gamma-point bare

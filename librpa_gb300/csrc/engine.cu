@@ -183,6 +183,7 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
         cudaStream_t s;
         ~StreamGuard() { cudaStreamDestroy(s); }
     } sg{st};
+    ArenaScope arena(st);
     long long launches = 0;
     const double t_up0 = wall_seconds();
     auto d_ao_off = to_dev(ao_off, st);
@@ -227,6 +228,7 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
                           din->vblob.size() == ds.vq_blob.size() && din->csblob.size() == n_cs;
         if (!fits)
         {
+            ArenaPause kept;  // these stay with the handler
             ds.dev_cache.reset();
             din.reset();
             din = std::make_shared<DeviceInputs>();
@@ -662,7 +664,7 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
         // keep the partial chi0(q, w) and stop before E_c
         release_kept(ds);
         ds.kept_chi0_bytes = d_chi0q.bytes();
-        GB_CUDA(cudaMalloc(&ds.kept_chi0, ds.kept_chi0_bytes));
+        ds.kept_chi0 = device_malloc(ds.kept_chi0_bytes);
         GB_CUDA(cudaMemcpyAsync(ds.kept_chi0, d_chi0q.get(), ds.kept_chi0_bytes, cudaMemcpyDeviceToDevice, st));
         ds.kept_pair_offset.assign(e_off.begin(), e_off.end());
         ds.kept_pair_elems = static_cast<size_t>(e_tot);
@@ -885,7 +887,7 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
         // complex M' is factored as its real 2N x 2N embedding: 32 bytes per element of M'
         const double per_q = static_cast<double>(nw) * NN * (gamma_only ? esz : 2 * esz) + NN * esz;
         const int qb = std::max(1, std::min(std::max(qe - qa, 1), static_cast<int>(24.0e9 / per_q)));
-        EcChol ecc(Ne, nw, !gamma_only, qb, go.ec_path == LIBRPA_GB300_EC_CHOL_FP64);
+        EcChol ecc(Ne, nw, !gamma_only, qb, go.ec_path == LIBRPA_GB300_EC_CHOL_FP64, st);
         DevBuf<unsigned char> Vall(static_cast<size_t>(qb) * NN * esz), X(static_cast<size_t>(nw) * NN * esz);
         for (int q0 = qa; q0 < qe; q0 += qb)
         {
@@ -937,7 +939,7 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
     if (go.keep_chi0 && go.stage == LIBRPA_GB300_STAGE_FULL)
     {
         ds.kept_chi0_bytes = d_chi0q.bytes();
-        GB_CUDA(cudaMalloc(&ds.kept_chi0, ds.kept_chi0_bytes));
+        ds.kept_chi0 = device_malloc(ds.kept_chi0_bytes);
         GB_CUDA(cudaMemcpyAsync(ds.kept_chi0, d_chi0q.get(), ds.kept_chi0_bytes, cudaMemcpyDeviceToDevice, st));
         ds.kept_pair_offset.assign(e_off.begin(), e_off.end());
         ds.kept_pair_elems = static_cast<size_t>(e_tot);

@@ -1050,6 +1050,7 @@ void build_exx(Dataset &ds, const LibrpaOptions &opts)
         cudaStream_t s;
         ~Guard() { cudaStreamDestroy(s); }
     } guard{st};
+    ArenaScope arena(st);
     GammaSetup gs;
     if (shrink)
     {
@@ -1151,6 +1152,7 @@ void build_g0w0_gamma(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
         cudaStream_t s;
         ~Guard() { cudaStreamDestroy(s); }
     } guard{st};
+    ArenaScope arena(st);
     GammaSetup gs;
     setup_gamma(ds, opts.libri_g0w0_threshold_C, gs, st);
     const int N = gs.N, nao = gs.nao, nb = ds.n_states, ns = ds.n_spins, nw = tf.n;
@@ -1358,6 +1360,7 @@ void build_g0w0_kgrid(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
         cudaStream_t s;
         ~Guard() { cudaStreamDestroy(s); }
     } guard{st};
+    ArenaScope arena(st);
     GammaSetup gs;
     setup_gamma(ds, opts.libri_g0w0_threshold_C, gs, st);
     const PhaseTables pt = build_phase_tables(ds);

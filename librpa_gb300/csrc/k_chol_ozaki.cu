@@ -309,32 +309,25 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 
 } // namespace
 
-void ozaki_alloc(OzakiWork &w, int N, int batch)
+void ozaki_alloc(OzakiWork &w, int N, int batch, cudaStream_t st)
 {
-    ozaki_free(w);
-    GB_CUDA(cudaMalloc(&w.slices, sizeof(__nv_bfloat16) * static_cast<size_t>(batch) * SL * N * OK));
-    GB_CUDA(cudaMalloc(&w.expo, sizeof(int) * static_cast<size_t>(batch) * N));
-    GB_CUDA(cudaMalloc(&w.err, sizeof(int)));
-    GB_CUDA(cudaMemset(w.err, 0, sizeof(int)));
-    GB_CUDA(cudaMalloc(&w.winv, sizeof(double) * static_cast<size_t>(batch) * OK * OK));
+    w = OzakiWork{};
+    auto buf = [&](size_t bytes) -> void * {
+        w.own.emplace_back(bytes);
+        return w.own.back().get();
+    };
     const size_t wsl = static_cast<size_t>(batch) * SL * 2 * OK * OK;
-    GB_CUDA(cudaMalloc(&w.wslices, sizeof(__nv_bfloat16) * wsl));
-    GB_CUDA(cudaMemset(w.wslices, 0, sizeof(__nv_bfloat16) * wsl));  // rows OK..2 OK stay zero
-    GB_CUDA(cudaMalloc(&w.wexpo, sizeof(int) * static_cast<size_t>(batch) * 2 * OK));
-    GB_CUDA(cudaMemset(w.wexpo, 0, sizeof(int) * static_cast<size_t>(batch) * 2 * OK));
+    w.slices = buf(sizeof(__nv_bfloat16) * static_cast<size_t>(batch) * SL * N * OK);
+    w.expo = static_cast<int *>(buf(sizeof(int) * static_cast<size_t>(batch) * N));
+    w.err = static_cast<int *>(buf(sizeof(int)));
+    w.winv = static_cast<double *>(buf(sizeof(double) * static_cast<size_t>(batch) * OK * OK));
+    w.wslices = buf(sizeof(__nv_bfloat16) * wsl);
+    w.wexpo = static_cast<int *>(buf(sizeof(int) * static_cast<size_t>(batch) * 2 * OK));
+    GB_CUDA(cudaMemsetAsync(w.err, 0, sizeof(int), st));
+    GB_CUDA(cudaMemsetAsync(w.wslices, 0, sizeof(__nv_bfloat16) * wsl, st));  // rows OK..2 OK stay zero
+    GB_CUDA(cudaMemsetAsync(w.wexpo, 0, sizeof(int) * static_cast<size_t>(batch) * 2 * OK, st));
     w.N = N;
     w.batch = batch;
-}
-
-void ozaki_free(OzakiWork &w)
-{
-    if (w.slices) cudaFree(w.slices);
-    if (w.expo) cudaFree(w.expo);
-    if (w.err) cudaFree(w.err);
-    if (w.winv) cudaFree(w.winv);
-    if (w.wslices) cudaFree(w.wslices);
-    if (w.wexpo) cudaFree(w.wexpo);
-    w = OzakiWork{};
 }
 
 namespace {
@@ -443,7 +436,7 @@ double chol_ozaki_selftest(int N, int batch, int seed, int spread_decades, doubl
     DevBuf<int> bad(batch);
     bad.zero(st);
     OzakiWork w;
-    ozaki_alloc(w, N, batch);
+    ozaki_alloc(w, N, batch, st);
     chol_batched_r(a1.get(), N, batch, d1.get(), bad.get(), st);
     chol_batched_r_ozaki(a2.get(), N, batch, d2.get(), bad.get(), w, st);
     chol_logdet(d1.get(), N, batch, l1.get(), st);
@@ -458,7 +451,6 @@ double chol_ozaki_selftest(int N, int batch, int seed, int spread_decades, doubl
     bad.download(hbad.data(), batch, st);
     GB_CUDA(cudaMemcpyAsync(&herr, w.err, sizeof(int), cudaMemcpyDeviceToHost, st));
     GB_CUDA(cudaStreamSynchronize(st));
-    ozaki_free(w);
     cudaStreamDestroy(st);
     GB_REQUIRE(herr == 0, "Ozaki update reported wait timeout code " + std::to_string(herr));
     for (int b = 0; b < batch; ++b) GB_REQUIRE(hbad[b] == 0, "test matrix not positive definite");
