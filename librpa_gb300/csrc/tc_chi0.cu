@@ -15,6 +15,8 @@
 //     the tcgen05.mma terms.  K order: 8-column chunk, group of 8 j.
 //  3. T2 (small, CUDA cores): D += sum_{i,j} X_b^I[mu i; (cJ,J) j] X_a^J[nu j; (-cJ,I) i].
 // Every wait is bounded (tc_common.cuh) and failures surface through a device error flag.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -49,6 +51,7 @@ constexpr int T1_ACOLS = NS * 32;                  // columns of one A tile: 3 p
 constexpr int T1_ABASE = T1_TMEM - 2 * T1_ACOLS;   // one A tile per producer warpgroup
 constexpr int T1_MAXA = 32;                        // max NAOs per atom
 constexpr int T1_CELLS = 32;                       // cells of a row group's shift table in shared memory
+constexpr int T1_INFO = 8;                         // ints kept of a row group: pair, cell, I, n_abf(I), n_ao(I)
 constexpr int T1_SMEM_MAX = 227 * 1024;
 // Shared memory: nbs x NS B pieces of b_tile bytes | X ring | G blocks | barriers.  b_tile = NT_max * 128
 // rounded up to 1024; a G block holds, per 8 j, the 2 n_ao(I) rows q = (pass, i).
@@ -75,7 +78,7 @@ struct T1Work
 
 constexpr int T1_MAXSPEC = 8;    // distinct (NAO, ABF) species with their own B maps
 constexpr int T1_KPARTS = 4;     // default K parts per tile (each part a CTA, added into chi0(R) atomically)
-constexpr int T1_KPARTS_MAX = 8; // largest K-part count the tuner tries
+constexpr int T1_KPARTS_MAX = 16; // largest K-part count the tuner tries
 
 // C^J B-operand maps, one rank-3 map per (species, piece): dims {ktot, nabf, atoms of the species}.
 struct T1Maps
@@ -110,11 +113,6 @@ struct T1Args
 __device__ __forceinline__ void named_bar_sync(int id, int n)
 {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
-}
-
-__device__ __forceinline__ uint32_t bf2_bits(__nv_bfloat162 h)
-{
-    return *reinterpret_cast<const uint32_t *>(&h);
 }
 
 // Three-piece BF16 split of a pair of FP32 values (hi, mid, lo), each piece packed as bf16x2
@@ -328,7 +326,7 @@ __global__ void __launch_bounds__(T1_THREADS, 1) k_t1_tc(const __grid_constant__
     const int gq = a.gq;                      // rows q of a G block's part of 8 j
     unsigned char *xring = bring + nbs * bstage_bytes;
     float *gsm = reinterpret_cast<float *>(xring + T1_XBYTES);
-    uint64_t *full = reinterpret_cast<uint64_t *>(gsm + a.maxcj * (a.gslot + T1_CELLS));  // [set][half] A tile: written
+    uint64_t *full = reinterpret_cast<uint64_t *>(gsm + a.maxcj * (a.gslot + T1_CELLS + T1_INFO));  // [set][half] A tile: written
     uint64_t *empty = full + 4;                                              // A tile: MMAs done
     uint64_t *bfull = empty + 4;                                             // B ring: TMA landed
     uint64_t *bempty = bfull + T1_MAXB;                                      // B ring: MMAs done
@@ -346,16 +344,31 @@ __global__ void __launch_bounds__(T1_THREADS, 1) k_t1_tc(const __grid_constant__
     const int NT = (bJ + 15) / 16 * 16;
     const int nab = 2 * NBLK * NT <= T1_ABASE ? 2 : 1;  // accumulator buffers
     const int nc = g.n_c, nao = g.n_ao;
-    // row r of the tile -> (row group, mu); false beyond the tile's valid rows
-    auto row_of = [&](int r, int &grp, int &mu) -> bool {
+    // the tile's row groups, read once (every later look at them would be a chain of global loads)
+    int *ctab = reinterpret_cast<int *>(gsm + a.maxcj * a.gslot);  // [slot][T1_CELLS]
+    int *info = ctab + a.maxcj * T1_CELLS;                         // [slot][T1_INFO]
+    if (threadIdx.x < static_cast<unsigned>(w.nslot))
+    {
+        const T1Group gr = a.groups[w.g0 + threadIdx.x];
+        const int Ig = a.pr.I[gr.pair];
+        int *f = info + threadIdx.x * T1_INFO;
+        f[0] = gr.pair;
+        f[1] = gr.cell;
+        f[2] = Ig;
+        f[3] = g.nabf[Ig];
+        f[4] = g.nao[Ig];
+    }
+    // row r of the tile -> (slot of its row group, mu); false beyond the tile's valid rows
+    auto row_of = [&](int r, int &slot, int &mu) -> bool {
+        slot = mu = 0;
         if (r >= w.nrows) return false;
-        int off = w.r0 + r, gi = w.g0;
-        for (int k = 0; k < w.nslot; ++k, ++gi)
+        int off = w.r0 + r;
+        for (int k = 0; k < w.nslot; ++k)
         {
-            const int b = g.nabf[a.pr.I[a.groups[gi].pair]];
+            const int b = info[k * T1_INFO + 3];
             if (off < b)
             {
-                grp = gi;
+                slot = k;
                 mu = off;
                 return true;
             }
@@ -399,39 +412,36 @@ __global__ void __launch_bounds__(T1_THREADS, 1) k_t1_tc(const __grid_constant__
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PREG));
         const int t = threadIdx.x;
         const int set = t / T1_SET;  // chunks kc0 + set, kc0 + set + 2, ...
-        int grp = w.g0, mu = 0;
-        const bool valid = row_of(t % T1_SET, grp, mu);
-        const int I = a.pr.I[a.groups[grp].pair];
-        const int cJ = a.groups[grp].cell;
-        const int aI = g.nao[I], bI = g.nabf[I];
+        int gslot, mu;
+        const bool valid = row_of(t % T1_SET, gslot, mu);
+        const int *mine = info + gslot * T1_INFO;
+        const int cJ = mine[1], I = mine[2], bI = mine[3], aI = mine[4];
         const float4 *xrow = a.Xt + a.xoff[I] + mu;
         // G blocks of the tile's row groups, [slot][j / 8][q = (pass, i)][j % 8] in FP32 (zero rows past
         // 2 a_I, zero past a_J)
-        const int nq = 2 * w.ra;
-        for (int s = 0; s < w.nslot; ++s)
+        const int nq = 2 * w.ra, per = njg * nq * JG;
+#pragma unroll 4
+        for (int x = t; x < w.nslot * per; x += T1_PRODUCERS)
         {
-            const T1Group gr = a.groups[w.g0 + s];
-            const int Ig = a.pr.I[gr.pair], ag = g.nao[Ig];
-            for (int e = t; e < njg * nq * JG; e += T1_PRODUCERS)
-            {
-                const int jg = e / (nq * JG), q = e / JG % nq, j = jg * JG + e % JG;
-                const int pass = q >= ag, i = pass ? q - ag : q;
-                float v = 0.0f;
-                if (q < 2 * ag && j < aJ)
-                    v = static_cast<float>(a.G[((static_cast<size_t>(pass) * nc + gr.cell) * nao + g.ao_off[Ig] + i) * nao +
-                                               g.ao_off[J] + j]);
-                gsm[s * a.gslot + (jg * gq + q) * JG + e % JG] = v;
-            }
+            const int s = x / per, e = x - s * per;
+            const int *f = info + s * T1_INFO;
+            const int Ig = f[2], ag = f[4];
+            const int jg = e / (nq * JG), q = e / JG % nq, j = jg * JG + e % JG;
+            const int pass = q >= ag, i = pass ? q - ag : q;
+            float v = 0.0f;
+            if (q < 2 * ag && j < aJ)
+                v = static_cast<float>(a.G[((static_cast<size_t>(pass) * nc + f[1]) * nao + g.ao_off[Ig] + i) * nao +
+                                           g.ao_off[J] + j]);
+            gsm[s * a.gslot + (jg * gq + q) * JG + e % JG] = v;
         }
         // cells of the shifted columns of each row group: R' + R_cJ (kept in shared memory for up to
         // T1_CELLS cells, read once per chunk)
-        int *ctab = reinterpret_cast<int *>(gsm + a.maxcj * a.gslot);
         if (nc <= T1_CELLS)
             for (int e = t; e < w.nslot * nc; e += T1_PRODUCERS)
-                ctab[e / nc * T1_CELLS + e % nc] = a.cadd[(e % nc) * nc + a.groups[w.g0 + e / nc].cell];
-        const int *crow = nc <= T1_CELLS ? ctab + (grp - w.g0) * T1_CELLS : nullptr;
+                ctab[e / nc * T1_CELLS + e % nc] = a.cadd[(e % nc) * nc + info[e / nc * T1_INFO + 1]];
+        const int *crow = nc <= T1_CELLS ? ctab + gslot * T1_CELLS : nullptr;
         named_bar_sync(1, T1_PRODUCERS);
-        const uint32_t gs = smem_u32(gsm + (grp - w.g0) * a.gslot);
+        const uint32_t gs = smem_u32(gsm + gslot * a.gslot);
         // units of j: all of an atom of 9 to 14 NAOs at once, 8 at a time otherwise (E of a thread's row
         // and chunk is 14 x 8 registers at most)
         const bool wide = JT == 16 && aJ > 8 && aJ <= 14;
@@ -698,12 +708,11 @@ __global__ void __launch_bounds__(T1_THREADS, 1) k_t1_tc(const __grid_constant__
             if (lane == 0) mbar_arrive(&acce[ab]);
             if (++ab == nab) ab = 0, ph ^= 1;
         }
-        int grp = 0, mu = 0;
-        if (ok && row_of(wq * 32 + lane, grp, mu))
+        int slot, mu;
+        if (row_of(wq * 32 + lane, slot, mu) && ok)
         {
-            const T1Group gr = a.groups[grp];
-            const int bI = g.nabf[a.pr.I[gr.pair]];
-            double *orow = a.out + a.pr.r_off[gr.pair] + (static_cast<long long>(gr.cell) * bI + mu) * bJ;
+            const int *f = info + slot * T1_INFO;
+            double *orow = a.out + a.pr.r_off[f[0]] + (static_cast<long long>(f[1]) * f[3] + mu) * bJ;
 #pragma unroll
             for (int c = 0; c < NTC; ++c)
                 if (c < bJ)
@@ -729,8 +738,11 @@ __global__ void __launch_bounds__(T1_THREADS, 1) k_t1_tc(const __grid_constant__
 // contiguous bytes.  A step takes 4 i x 4 j: one float4 of each operand per thread, transposed through
 // shared memory to [k = (i, j)][mu] and [k][nu] without bank conflicts, the next step's loads in flight
 // meanwhile; each of the tile's (mu, nu) 4 x 4 blocks is one thread's.  Bound by the latency of its steps
-// in small cells and by the FP32 pipe in large ones.  Tiles are disjoint and the CTA sums both passes
-// before its one add, so the result does not depend on CTA order.
+// in small cells and by the FP32 pipe in large ones.  Where the tiles leave SMs idle, the steps of one are
+// dealt to a cluster of CTAs (z), whose first sums the parts in order through distributed shared memory.
+// Tiles are disjoint and each is added once, so the result does not depend on CTA order.  One GB300, a
+// launch: 3 atoms of 5/20, 13/60, 26/110 at Gamma 283 -> 107 us by the steps, 42 by the parts; 128 atoms of
+// 13/40 1.77 -> 0.73 ms.
 constexpr int T2_THREADS = 256;
 constexpr int T2_TILE = 64;
 
@@ -738,7 +750,8 @@ __global__ void __launch_bounds__(T2_THREADS) k_t2(const float4 *__restrict__ Xt
                                                   Geom g, Pairs pr, const T1Group *__restrict__ groups, int tiles,
                                                   double *__restrict__ out)
 {
-    __shared__ __align__(16) float S1[2][16][T2_TILE], S2[2][16][T2_TILE];
+    __shared__ __align__(16) float buf[2][2][16][T2_TILE];  // [operand][step parity][k][row]; the parts' sum
+    auto &S1 = buf[0], &S2 = buf[1];
     const int p = groups[blockIdx.x].pair, cJ = groups[blockIdx.x].cell;
     const int I = pr.I[p], J = pr.J[p];
     const int aI = g.nao[I], aJ = g.nao[J], bI = g.nabf[I], bJ = g.nabf[J];
@@ -748,6 +761,8 @@ __global__ void __launch_bounds__(T2_THREADS) k_t2(const float4 *__restrict__ Xt
     // first column group of each atom and the atom's first column inside it
     const int gI = g.ao_off[I] / 4, sI = g.ao_off[I] % 4, gJ = g.ao_off[J] / 4, sJ = g.ao_off[J] % 4;
     const int nI = (sI + aI + 3) / 4, nJ = (sJ + aJ + 3) / 4, steps = 2 * nI * nJ;
+    const int nsplit = static_cast<int>(gridDim.z), part = static_cast<int>(blockIdx.z);
+    const int st0 = steps * part / nsplit, st1 = steps * (part + 1) / nsplit;
     const int r = threadIdx.x % T2_TILE, s = threadIdx.x / T2_TILE;  // staging: row and i (or j) of the step
     const long long rI = static_cast<long long>(t1_rows(aI)) * bI, rJ = static_cast<long long>(t1_rows(aJ)) * bJ;
     const float4 *XI = Xt + xoff[I] + (static_cast<long long>(cJ) * n4 + gJ) * rI + mt0 + r;
@@ -768,14 +783,14 @@ __global__ void __launch_bounds__(T2_THREADS) k_t2(const float4 *__restrict__ Xt
 #pragma unroll
     for (int a = 0; a < 4; ++a) acc[a][0] = acc[a][1] = make_float2(0.f, 0.f);
     float4 v1, v2;
-    load(0, v1, v2);
-    for (int st = 0; st < steps; ++st)
+    load(min(st0, steps - 1), v1, v2);
+    for (int st = st0; st < st1; ++st)
     {
         float(*A)[T2_TILE] = S1[st & 1], (*B)[T2_TILE] = S2[st & 1];
         A[4 * s][r] = v1.x, A[4 * s + 1][r] = v1.y, A[4 * s + 2][r] = v1.z, A[4 * s + 3][r] = v1.w;
         B[s][r] = v2.x, B[4 + s][r] = v2.y, B[8 + s][r] = v2.z, B[12 + s][r] = v2.w;
         __syncthreads();
-        if (st + 1 < steps) load(st + 1, v1, v2);
+        if (st + 1 < st1) load(st + 1, v1, v2);
         if (live)
         {
             // the i and j of this step that lie inside the atoms
@@ -801,16 +816,36 @@ __global__ void __launch_bounds__(T2_THREADS) k_t2(const float4 *__restrict__ Xt
                 }
         }
     }
-    if (!live) return;
     double *o = out + pr.r_off[p] + static_cast<long long>(cJ) * bI * bJ + static_cast<long long>(mt0 + m0) * bJ + nt0 + n0;
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
+    float *tile = &buf[0][0][0][0];  // [T2_TILE][T2_TILE] of a part
+    static_assert(sizeof(buf) >= sizeof(float) * T2_TILE * T2_TILE, "a part's tile fits the staging buffers");
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    if (nsplit > 1)
     {
-        const float v[4] = {acc[a][0].x, acc[a][0].y, acc[a][1].x, acc[a][1].y};
+        __syncthreads();
+        if (live && part != 0)
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-            if (m0 + a < mn && n0 + c < nn) o[static_cast<long long>(a) * bJ + c] += static_cast<double>(v[c]);
+            for (int a = 0; a < 4; ++a)
+                *reinterpret_cast<float4 *>(tile + (m0 + a) * T2_TILE + n0) =
+                    make_float4(acc[a][0].x, acc[a][0].y, acc[a][1].x, acc[a][1].y);
+        cl.sync();
     }
+    if (live && part == 0)
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+        {
+            const float v[4] = {acc[a][0].x, acc[a][0].y, acc[a][1].x, acc[a][1].y};
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (m0 + a < mn && n0 + c < nn)
+                {
+                    double x = static_cast<double>(v[c]);
+                    for (int k = 1; k < nsplit; ++k)
+                        x += static_cast<double>(cl.map_shared_rank(tile, k)[(m0 + a) * T2_TILE + n0 + c]);
+                    o[static_cast<long long>(a) * bJ + c] += x;
+                }
+        }
+    if (nsplit > 1) cl.sync();  // the tiles stay until they are read
 }
 
 // B operand of X = C * Gs: row n = (cL, l), column k = (cK, k'):  Gs^T[n][k] = G[cdiff(cL,cK)][k'][l]
@@ -1096,7 +1131,7 @@ TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st)
     m.gslot = m.gq * ((g.max_nao + JG - 1) / JG * JG) + 4;
     // shared memory: at least two B stages + the G slots; fewer G slots than a tile of small row
     // groups could touch only shortens such tiles
-    const int slot_bytes = (m.gslot + T1_CELLS) * 4;
+    const int slot_bytes = (m.gslot + T1_CELLS + T1_INFO) * 4;
     const int base = 1024 + T1_XBYTES + 512;
     const int fit = (T1_SMEM_MAX - base - 2 * NS * m.b_tile) / slot_bytes;
     GB_REQUIRE(fit >= 1, "chi0 tile does not fit shared memory (too many ABFs or NAOs per atom)");
@@ -1123,7 +1158,7 @@ TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st)
             const std::string lay = v.substr(0, c);
             const int kp = std::atoi(v.c_str() + c + 1);
             GB_REQUIRE((lay == "narrow" || lay == "wide") && kp >= 1 && kp <= T1_KPARTS_MAX,
-                       "LIBRPA_GB300_T1_LAUNCH must read narrow:<kparts> or wide:<kparts>, kparts 1-8");
+                       "LIBRPA_GB300_T1_LAUNCH must read narrow:<kparts> or wide:<kparts>, kparts 1-16");
             m.kparts = kp;
             m.kparts_forced = true;
             m.tuned = true;
@@ -1182,10 +1217,10 @@ void TcChi0::Impl::autotune(const double *G, double *chi0R, cudaStream_t st)
     GB_CUDA(cudaEventCreate(&e0));
     GB_CUDA(cudaEventCreate(&e1));
     T1Choice best{kparts, 1e30};
-    const int kp_cand[] = {1, 2, 4, 8};
+    const int kp_cand[] = {1, 2, 4, 8, 16};
     for (int kp : kp_cand)
     {
-        if (kp > T1_KPARTS_MAX || (kp > 1 && nkc < 2 * kp)) continue;
+        if (kp > T1_KPARTS_MAX || kp > nkc) continue;
         kparts = kp;
         kparts_forced = true;
         all_active = false;
@@ -1343,9 +1378,24 @@ int TcChi0::contract(const double *G, double *chi0R, const unsigned char *active
         {
             m.launch_t1(a, st);
             const int tiles = (g.max_nabf + T2_TILE - 1) / T2_TILE;
-            k_t2<<<dim3(m.n_groups, tiles * tiles), T2_THREADS, 0, st>>>(m.Xt.get(), m.xoff.get(), m.n4, g, m.pr,
-                                                                       m.groups.get(), tiles, chi0R);
-            GB_LAUNCH_CHECK();
+            // parts of a tile's steps while the tiles leave SMs idle, up to the portable cluster size; by the
+            // tiles of all blocks, so that a screened call sums a block as the unscreened one does
+            const long long ctas = static_cast<long long>(m.pr.n_pairs) * g.n_c * tiles * tiles;
+            const unsigned nsplit = static_cast<unsigned>(std::max<long long>(1, std::min<long long>(8, m.n_sm / ctas)));
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(m.n_groups, tiles * tiles, nsplit);
+            cfg.blockDim = dim3(T2_THREADS);
+            cfg.stream = st;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = 1;
+            at[0].val.clusterDim.y = 1;
+            at[0].val.clusterDim.z = nsplit;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            GB_CUDA(cudaLaunchKernelEx(&cfg, k_t2, static_cast<const float4 *>(m.Xt.get()),
+                                       static_cast<const long long *>(m.xoff.get()), m.n4, g, m.pr,
+                                       static_cast<const T1Group *>(m.groups.get()), tiles, chi0R));
             launches += 2;
         }
     }

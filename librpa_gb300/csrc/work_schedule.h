@@ -141,7 +141,7 @@ inline std::vector<KPart> plan_kparts(int n_tiles, int n_sm, int nkc, int kparts
     std::vector<KPart> out;
     const int kparts =
         force || static_cast<long long>(n_tiles) < 16LL * (n_sm > 0 ? n_sm : 1) ? kparts_max : 1;
-    const bool cut = kparts > 1 && nkc >= 2 * kparts;
+    const bool cut = kparts > 1 && nkc >= (force ? 1 : 2) * kparts;  // a forced count was timed
     for (int t = 0; t < n_tiles; ++t)
     {
         if (!cut)
