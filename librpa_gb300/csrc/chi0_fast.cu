@@ -51,6 +51,11 @@ Chi0Fast::~Chi0Fast() = default;
 
 TcChi0 *Chi0Fast::tensor_path() { return impl_->tc.get(); }
 
+void Chi0Fast::check(cudaStream_t st) const
+{
+    if (impl_->tc) impl_->tc->check(st);
+}
+
 int Chi0Fast::run(const double *Gs, const double *Gp, const double *Gm, double *chi0R, cudaStream_t st)
 {
     Impl &m = *impl_;

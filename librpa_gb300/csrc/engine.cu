@@ -40,28 +40,42 @@ namespace gb {
 
 namespace {
 
-struct EventTimer
+// Device time of the spans between start() and stop(), summed by total_ms() at the end: reading a span as
+// it closes would stop the host after every stage.
+class EventTimer
 {
-    cudaEvent_t a = nullptr, b = nullptr;
-    EventTimer()
-    {
-        GB_CUDA(cudaEventCreate(&a));
-        GB_CUDA(cudaEventCreate(&b));
-    }
+public:
+    EventTimer() = default;
+    EventTimer(const EventTimer &) = delete;
+    EventTimer &operator=(const EventTimer &) = delete;
     ~EventTimer()
     {
-        if (a) cudaEventDestroy(a);
-        if (b) cudaEventDestroy(b);
+        for (cudaEvent_t e : ev_) cudaEventDestroy(e);
     }
-    void start(cudaStream_t s) { GB_CUDA(cudaEventRecord(a, s)); }
-    void stop(cudaStream_t s) { GB_CUDA(cudaEventRecord(b, s)); }
-    double ms()
+    void start(cudaStream_t s) { record(s); }
+    void stop(cudaStream_t s) { record(s); }
+    double total_ms()
     {
-        GB_CUDA(cudaEventSynchronize(b));
-        float t = 0;
-        GB_CUDA(cudaEventElapsedTime(&t, a, b));
-        return t;
+        double sum = 0.0;
+        for (size_t i = 0; i + 1 < ev_.size(); i += 2)
+        {
+            GB_CUDA(cudaEventSynchronize(ev_[i + 1]));
+            float t = 0;
+            GB_CUDA(cudaEventElapsedTime(&t, ev_[i], ev_[i + 1]));
+            sum += t;
+        }
+        return sum;
     }
+
+private:
+    void record(cudaStream_t s)
+    {
+        cudaEvent_t e = nullptr;
+        GB_CUDA(cudaEventCreate(&e));
+        ev_.push_back(e);
+        GB_CUDA(cudaEventRecord(e, s));
+    }
+    std::vector<cudaEvent_t> ev_;  // start, stop, start, stop ...
 };
 
 } // namespace
@@ -359,7 +373,11 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
     double ftct_bytes = 0.0;
     DevBuf<cuDoubleComplex> d_chi0q(static_cast<size_t>(nw) * nq * e_tot);
     d_chi0q.zero(st);
-    DevBuf<double> d_gamma(static_cast<size_t>(nw));
+    // the cosine transform's columns, [tau][omega]
+    std::vector<double> h_gamma(static_cast<size_t>(nw) * nw);
+    for (int it = 0; it < nw; ++it)
+        for (int w = 0; w < nw; ++w) h_gamma[static_cast<size_t>(it) * nw + w] = tf.cos_t2f[static_cast<size_t>(w) * nw + it];
+    auto d_gamma = to_dev(h_gamma, st);
 
     std::unique_ptr<Chi0Fast> fast;
     if (prec != LIBRPA_GB300_CHI0_FP64) fast = std::make_unique<Chi0Fast>(prec, g, pr, d_C.get(), st);
@@ -440,7 +458,6 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
     }
 
     EventTimer ev_gf, ev_x, ev_chi, ev_ft;
-    double t_gf = 0, t_chi = 0, t_ft = 0;
     double flops_chi = 0.0, flops_libri = 0.0;
     S.dt_chi0_kernel_ms = 0.0;
     S.n_chi0_kernel = 0;
@@ -459,9 +476,7 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
     for (int it = do_chi0 ? tb : te; it < te; ++it)
     {
         const double tau = tf.tau[it];
-        std::vector<double> gam(nw);
-        for (int w = 0; w < nw; ++w) gam[w] = tf.cos_t2f[static_cast<size_t>(w) * nw + it];
-        d_gamma.upload(gam.data(), nw, st);
+        const double *gam = h_gamma.data() + static_cast<size_t>(it) * nw;
         for (int is = 0; is < ns; ++is)
         {
             double *chi0R_cur = batch_ft ? d_slots.get() + static_cast<size_t>(slots_filled) * r_tot : d_chi0R.get();
@@ -488,7 +503,6 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
                 ++launches;
             }
             ev_gf.stop(st);
-            t_gf += ev_gf.ms();
             ev_chi.start(st);
             const double *Gp = d_G.get(), *Gm = d_G.get() + static_cast<size_t>(nc) * nao * nao;
             if (prec == LIBRPA_GB300_CHI0_FP64)
@@ -572,8 +586,6 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
                 ++launches;
             }
             ev_chi.stop(st);
-            t_chi += ev_chi.ms();
-            S.dt_chi0_kernel_ms += ev_x.ms();
             S.n_chi0_kernel += 1;
             ev_ft.start(st);
             if (batch_ft)
@@ -599,12 +611,12 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
             }
             else
             {
-                launch_ftct(chi0R_cur, g, pr, d_qcos.get(), d_qsin.get(), nq, d_gamma.get(), nw, fac, d_chi0q.get(), st);
+                launch_ftct(chi0R_cur, g, pr, d_qcos.get(), d_qsin.get(), nq,
+                            d_gamma.get() + static_cast<size_t>(it) * nw, nw, fac, d_chi0q.get(), st);
                 ++launches;
                 ftct_bytes += 8.0 * r_tot + 2.0 * 16.0 * nw * nq * e_tot;
             }
             ev_ft.stop(st);
-            t_ft += ev_ft.ms();
         }
     }
     // FLOP counts per tau and spin.
@@ -640,6 +652,7 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
         d_err.download(&herr, 1, st);
         GB_CUDA(cudaStreamSynchronize(st));
         GB_REQUIRE(herr == 0, "tensor-core G build reported wait timeout code " + std::to_string(herr));
+        if (fast) fast->check(st);
     }
     if (TcChi0 *tp = fast ? fast->tensor_path() : nullptr)
     {
@@ -648,9 +661,10 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
         S.t1_narrow = nar;
         S.t1_kparts = kp;
     }
-    S.t_gf = t_gf * 1e-3;
-    S.t_chi0 = t_chi * 1e-3;
-    S.t_ftct = t_ft * 1e-3;
+    S.t_gf = ev_gf.total_ms() * 1e-3;
+    S.t_chi0 = ev_chi.total_ms() * 1e-3;
+    S.t_ftct = ev_ft.total_ms() * 1e-3;
+    S.dt_chi0_kernel_ms = ev_x.total_ms();
     S.chi0_flops = flops_chi;
     S.chi0_flops_libri = flops_libri;
     S.gf_flops = static_cast<double>(do_chi0 ? te - tb : 0) * ns * 2.0 * (8.0 * nk * nao * nao * nb + 4.0 * nc * nk * nao * nao);
@@ -781,67 +795,49 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
                    go.ec_path == LIBRPA_GB300_EC_CHOL_FP64,
                "unknown ec_path " + std::to_string(go.ec_path));
     const bool use_chol = go.ec_path != LIBRPA_GB300_EC_LU_FP64;
-    // V(q) from the blocks of this q inside the staged Coulomb blob
-    auto assemble_v = [&](int q, void *V) {
-        std::vector<long long> voff;
-        std::vector<int> vIJ;
+    // the Coulomb blocks of this call's q inside the staged blob: offset, and atoms I, J
+    std::vector<long long> voff;
+    std::vector<int> vIJ;
+    std::vector<size_t> vfirst(nq + 1, 0);
+    for (int q = 0; q < nq; ++q)
+    {
         for (int bi : vq_of_q[q])
         {
             const VqBlock &b = ds.vq_blocks[bi];
-            GB_REQUIRE(b.nmu == nabf_e[b.I] && b.nnu == nabf_e[b.J], "Coulomb block dimensions inconsistent");
+            GB_REQUIRE(q < qa || q >= qe || (b.nmu == nabf_e[b.I] && b.nnu == nabf_e[b.J]), "Coulomb block dimensions inconsistent");
             voff.push_back(static_cast<long long>(b.offset));
             vIJ.push_back(b.I);
             vIJ.push_back(b.J);
         }
-        auto d_voff = to_dev(voff, st);
-        auto d_vIJ = to_dev(vIJ, st);
-        if (gamma_only)
-        {
-            GB_CUDA(cudaMemsetAsync(V, 0, sizeof(double) * NN, st));
-            launch_assemble_v(din->vblob.get(), d_voff.get(), d_vIJ.get(), static_cast<int>(voff.size()), abf_off_e,
-                              nabf_dev_e, Ne, true, nullptr, static_cast<double *>(V), st);
-        }
-        else
-        {
-            GB_CUDA(cudaMemsetAsync(V, 0, sizeof(cuDoubleComplex) * NN, st));
-            launch_assemble_v(din->vblob.get(), d_voff.get(), d_vIJ.get(), static_cast<int>(voff.size()), abf_off_e,
-                              nabf_dev_e, Ne, false, static_cast<cuDoubleComplex *>(V), nullptr, st);
-        }
-        GB_CUDA(cudaStreamSynchronize(st));  // the block tables go out of scope
+        vfirst[q + 1] = voff.size();
+    }
+    auto d_voff = to_dev(voff, st);
+    auto d_vIJ = to_dev(vIJ, st);
+    // V(q) in full from its blocks, real at the Gamma point
+    auto assemble_v = [&](int q, void *V) {
+        const int n = static_cast<int>(vfirst[q + 1] - vfirst[q]);
+        GB_CUDA(cudaMemsetAsync(V, 0, (gamma_only ? sizeof(double) : sizeof(cuDoubleComplex)) * NN, st));
+        launch_assemble_v(din->vblob.get(), d_voff.get() + vfirst[q], d_vIJ.get() + 2 * vfirst[q], n, abf_off_e, nabf_dev_e,
+                          Ne, gamma_only, gamma_only ? nullptr : static_cast<cuDoubleComplex *>(V),
+                          gamma_only ? static_cast<double *>(V) : nullptr, st);
         ++launches;
     };
     // Reference form for one q: Pi = V chi0 in FP64, LU with partial pivoting, sum log(+-u_ii)
     // + tr Pi (epsilon.cpp:414-536).  It needs no definiteness of V(q).
     auto ec_lu_q = [&](int q)
     {
-        // V(q) full: blocks of this q inside the staged Coulomb blob
-        std::vector<long long> voff;
-        std::vector<int> vIJ;
-        for (int bi : vq_of_q[q])
-        {
-            const VqBlock &b = ds.vq_blocks[bi];
-            GB_REQUIRE(b.nmu == nabf_e[b.I] && b.nnu == nabf_e[b.J], "Coulomb block dimensions inconsistent");
-            voff.push_back(static_cast<long long>(b.offset));
-            vIJ.push_back(b.I);
-            vIJ.push_back(b.J);
-        }
-        auto d_voff = to_dev(voff, st);
-        auto d_vIJ = to_dev(vIJ, st);
-        const cuDoubleComplex *vbase = din->vblob.get();
         std::vector<double> tr_h(gamma_only ? nw : 2 * nw), ld_h(gamma_only ? nw : 2 * nw);
         if (gamma_only)
         {
             DevBuf<double> V(NN), X(NN * nw), P(NN * nw), tr(nw), ld(nw);
-            V.zero(st);
-            launch_assemble_v(vbase, d_voff.get(), d_vIJ.get(), static_cast<int>(voff.size()), abf_off_e,
-                              nabf_dev_e, Ne, true, nullptr, V.get(), st);
+            assemble_v(q, V.get());
             launch_assemble_chi0(chi0_e + static_cast<long long>(q) * e_tot_e, static_cast<long long>(nq) * e_tot_e, nw, Ne,
                                  atom_of_e, abf_off_e, nabf_dev_e, d_pair_of.get(), n_at, eoff_e, true,
                                  nullptr, X.get(), NN, st);
             launch_dgemm(Ne, Ne, Ne, V.get(), Ne, 0, X.get(), Ne, NN, P.get(), Ne, NN, nw, 1.0, 0.0, st);
             launch_trace_and_negate_r(P.get(), Ne, nw, tr.get(), st);
             launch_lu_logdet_r(P.get(), Ne, nw, ld.get(), st);
-            launches += 5;
+            launches += 4;
             tr.download(tr_h.data(), nw, st);
             ld.download(ld_h.data(), nw, st);
             GB_CUDA(cudaStreamSynchronize(st));
@@ -855,16 +851,14 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
         else
         {
             DevBuf<cuDoubleComplex> V(NN), X(NN * nw), P(NN * nw), tr(nw), ld(nw);
-            V.zero(st);
-            launch_assemble_v(vbase, d_voff.get(), d_vIJ.get(), static_cast<int>(voff.size()), abf_off_e,
-                              nabf_dev_e, Ne, false, V.get(), nullptr, st);
+            assemble_v(q, V.get());
             launch_assemble_chi0(chi0_e + static_cast<long long>(q) * e_tot_e, static_cast<long long>(nq) * e_tot_e, nw, Ne,
                                  atom_of_e, abf_off_e, nabf_dev_e, d_pair_of.get(), n_at, eoff_e, false,
                                  X.get(), nullptr, NN, st);
             launch_zgemm(Ne, Ne, Ne, V.get(), Ne, 0, X.get(), Ne, NN, P.get(), Ne, NN, nw, st);
             launch_trace_and_negate_c(P.get(), Ne, nw, tr.get(), st);
             launch_lu_logdet_c(P.get(), Ne, nw, ld.get(), st);
-            launches += 5;
+            launches += 4;
             tr.download(reinterpret_cast<cuDoubleComplex *>(tr_h.data()), nw, st);
             ld.download(reinterpret_cast<cuDoubleComplex *>(ld_h.data()), nw, st);
             GB_CUDA(cudaStreamSynchronize(st));
@@ -929,7 +923,7 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
     }
     for (int q = qa; q < qe && !use_chol; ++q) ec_lu_q(q);
     ev_ec.stop(st);
-    S.t_ec = ev_ec.ms() * 1e-3;
+    S.t_ec = ev_ec.total_ms() * 1e-3;
     S.ec_flops = ec_flops;
     S.ec_lu_fallback_q = lu_fallback_q;
     for (const cplx &v : res.per_q) res.ec += v;

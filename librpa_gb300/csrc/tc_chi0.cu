@@ -1399,11 +1399,15 @@ int TcChi0::contract(const double *G, double *chi0R, const unsigned char *active
             launches += 2;
         }
     }
+    return launches;
+}
+
+void TcChi0::check(cudaStream_t st) const
+{
     int herr = 0;
-    m.err.download(&herr, 1, st);
+    impl_->err.download(&herr, 1, st);
     GB_CUDA(cudaStreamSynchronize(st));
     GB_REQUIRE(herr == 0, "tensor-core chi0 kernel reported wait timeout code " + std::to_string(herr));
-    return launches;
 }
 
 } // namespace gb

@@ -97,6 +97,8 @@ public:
     // [pair * n_cells + cell], nullptr = all).  zero_first clears chi0R first, so blocks left
     // out read zero; a later call with zero_first = false adds further blocks.
     int contract(const double *G, double *chi0R, const unsigned char *active, bool zero_first, cudaStream_t st);
+    // Waits for the stream and throws if a kernel of prepare() or contract() gave up a wait.
+    void check(cudaStream_t st) const;
     // The contraction's launch choice: K parts per tile (narrow: always 0, there is one producer layout).
     void launch_choice(int &narrow, int &kparts) const;
 
