@@ -271,6 +271,10 @@ double librpa_gb300_selftest_tc_gemm(int M, int N, int K, int seed, int pieces);
  * max |L difference| / max |L|. */
 double librpa_gb300_selftest_chol_ozaki(int N, int batch, int seed, int spread_decades, double shift,
                                         double *max_rel_l);
+/* No counterpart in the reference.  The two forms of the FP64 LU log-determinant on `batch` random
+ * N x N matrices (kind 0: uniform entries, 1: entries -1, 0 and 1, 2: uniform with one NaN): the largest
+ * difference, infinite where only one form gives NaN; NaN on error. */
+double librpa_gb300_selftest_lu(int N, int batch, int is_complex, int kind, int seed);
 
 /* No counterpart in the reference.  D = A * B through the tcgen05 split-precision GEMM
  * (pieces = 2 or 3, as above) without allocating device memory, for callers that cannot

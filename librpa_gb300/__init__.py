@@ -144,6 +144,7 @@ EXPORTS = [
     "librpa_gb300_set_screening_model",
     "librpa_gb300_clear_screening", "librpa_gb300_mlp_loss_grad", "librpa_gb300_chi0_qw_elems",
     "librpa_gb300_copy_chi0_qw", "librpa_gb300_load_chi0_qw", "librpa_gb300_selftest_chol_ozaki",
+    "librpa_gb300_selftest_lu",
     "librpa_gb300_solve_qpe", "librpa_gb300_phase_tables", "librpa_gb300_interpolate_dielec_func",
 ]
 
@@ -214,6 +215,7 @@ def load_library(path: str | Path | None = None):
         "librpa_gb300_device_count": (i, []),
         "librpa_gb300_selftest_tc_gemm": (d, [i, i, i, i, i]),
         "librpa_gb300_selftest_chol_ozaki": (d, [i, i, i, i, d, C.POINTER(C.c_double)]),
+        "librpa_gb300_selftest_lu": (d, [i, i, i, i, i]),
         "librpa_gb300_tc_gemm_noalloc": (i, [i, i, i, C.c_void_p, C.c_void_p, C.c_void_p, i,
                                              C.c_void_p]),
         "librpa_gb300_train_screening": (i, [vp, i, d, C.POINTER(C.c_double)]),

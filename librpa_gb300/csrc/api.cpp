@@ -1339,6 +1339,17 @@ double librpa_gb300_selftest_chol_ozaki(int N, int batch, int seed, int spread_d
     return r;
 }
 
+double librpa_gb300_selftest_lu(int N, int batch, int is_complex, int kind, int seed)
+{
+    double r = std::numeric_limits<double>::quiet_NaN();
+    guarded(nullptr, [&] {
+        GB_REQUIRE(gb::device_count() > 0, "no CUDA device visible");
+        GB_REQUIRE(N > 0 && batch > 0, "N and batch must be positive");
+        r = gb::lu_selftest(N, batch, is_complex != 0, kind, seed);
+    });
+    return r;
+}
+
 // ---- kept chi0(q, omega) for tau-shard reductions; no counterpart in the reference
 long long librpa_gb300_chi0_qw_elems(LibrpaHandler *h)
 {

@@ -822,56 +822,59 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
                           gamma_only ? static_cast<double *>(V) : nullptr, st);
         ++launches;
     };
-    // Reference form for one q: Pi = V chi0 in FP64, LU with partial pivoting, sum log(+-u_ii)
-    // + tr Pi (epsilon.cpp:414-536).  It needs no definiteness of V(q).
-    auto ec_lu_q = [&](int q)
+    // Reference form for some q: Pi = V chi0 in FP64, LU with partial pivoting, sum log(+-u_ii)
+    // + tr Pi (epsilon.cpp:414-536).  It needs no definiteness of V(q).  The I - Pi of as many q as
+    // about 4 GB hold are factored by one launch: a few matrices leave the device idle.
+    auto ec_lu = [&](const std::vector<int> &qs)
     {
-        std::vector<double> tr_h(gamma_only ? nw : 2 * nw), ld_h(gamma_only ? nw : 2 * nw);
-        if (gamma_only)
+        if (qs.empty()) return;
+        const size_t comp = gamma_only ? 1 : 2;  // doubles per element
+        const int qb = std::max(1, std::min(static_cast<int>(qs.size()), static_cast<int>(4.0e9 / (8.0 * comp * NN * nw))));
+        DevBuf<double> V(comp * NN), X(comp * NN * nw), P(comp * NN * nw * qb), tr(comp * nw * qb), ld(comp * nw * qb);
+        std::vector<double> tr_h(comp * nw * qb), ld_h(comp * nw * qb);
+        const auto z = [](double *p) { return reinterpret_cast<cuDoubleComplex *>(p); };
+        for (size_t s0 = 0; s0 < qs.size(); s0 += qb)
         {
-            DevBuf<double> V(NN), X(NN * nw), P(NN * nw), tr(nw), ld(nw);
-            assemble_v(q, V.get());
-            launch_assemble_chi0(chi0_e + static_cast<long long>(q) * e_tot_e, static_cast<long long>(nq) * e_tot_e, nw, Ne,
-                                 atom_of_e, abf_off_e, nabf_dev_e, d_pair_of.get(), n_at, eoff_e, true,
-                                 nullptr, X.get(), NN, st);
-            launch_dgemm(Ne, Ne, Ne, V.get(), Ne, 0, X.get(), Ne, NN, P.get(), Ne, NN, nw, 1.0, 0.0, st);
-            launch_trace_and_negate_r(P.get(), Ne, nw, tr.get(), st);
-            launch_lu_logdet_r(P.get(), Ne, nw, ld.get(), st);
-            launches += 4;
-            tr.download(tr_h.data(), nw, st);
-            ld.download(ld_h.data(), nw, st);
-            GB_CUDA(cudaStreamSynchronize(st));
-            for (int w = 0; w < nw; ++w)
+            const int nb = static_cast<int>(std::min<size_t>(qb, qs.size() - s0));
+            for (int s = 0; s < nb; ++s)
             {
-                const cplx v = cplx(tr_h[w] + ld_h[w], 0.0) * tf.omega_w[w] * ibz_w[q] / (2.0 * M_PI);
-                res.per_q[q] += v;
+                const int q = qs[s0 + s];
+                double *Pq = P.get() + comp * NN * nw * s;
+                assemble_v(q, V.get());
+                launch_assemble_chi0(chi0_e + static_cast<long long>(q) * e_tot_e, static_cast<long long>(nq) * e_tot_e, nw, Ne,
+                                     atom_of_e, abf_off_e, nabf_dev_e, d_pair_of.get(), n_at, eoff_e, gamma_only,
+                                     gamma_only ? nullptr : z(X.get()), gamma_only ? X.get() : nullptr, NN, st);
+                if (gamma_only)
+                    launch_dgemm(Ne, Ne, Ne, V.get(), Ne, 0, X.get(), Ne, NN, Pq, Ne, NN, nw, 1.0, 0.0, st);
+                else
+                    launch_zgemm(Ne, Ne, Ne, z(V.get()), Ne, 0, z(X.get()), Ne, NN, z(Pq), Ne, NN, nw, st);
+                launches += 2;
             }
-            ec_flops += nw * (2.0 * Ne * Ne * Ne + 2.0 * Ne * Ne * Ne / 3.0);
-        }
-        else
-        {
-            DevBuf<cuDoubleComplex> V(NN), X(NN * nw), P(NN * nw), tr(nw), ld(nw);
-            assemble_v(q, V.get());
-            launch_assemble_chi0(chi0_e + static_cast<long long>(q) * e_tot_e, static_cast<long long>(nq) * e_tot_e, nw, Ne,
-                                 atom_of_e, abf_off_e, nabf_dev_e, d_pair_of.get(), n_at, eoff_e, false,
-                                 X.get(), nullptr, NN, st);
-            launch_zgemm(Ne, Ne, Ne, V.get(), Ne, 0, X.get(), Ne, NN, P.get(), Ne, NN, nw, st);
-            launch_trace_and_negate_c(P.get(), Ne, nw, tr.get(), st);
-            launch_lu_logdet_c(P.get(), Ne, nw, ld.get(), st);
-            launches += 4;
-            tr.download(reinterpret_cast<cuDoubleComplex *>(tr_h.data()), nw, st);
-            ld.download(reinterpret_cast<cuDoubleComplex *>(ld_h.data()), nw, st);
-            GB_CUDA(cudaStreamSynchronize(st));
-            for (int w = 0; w < nw; ++w)
+            if (gamma_only)
             {
-                const cplx v = (cplx(tr_h[2 * w], tr_h[2 * w + 1]) + cplx(ld_h[2 * w], ld_h[2 * w + 1])) *
-                               tf.omega_w[w] * ibz_w[q] / (2.0 * M_PI);
-                res.per_q[q] += v;
+                launch_trace_and_negate_r(P.get(), Ne, nw * nb, tr.get(), st);
+                launch_lu_logdet_r(P.get(), Ne, nw * nb, ld.get(), st);
             }
-            ec_flops += nw * (8.0 * Ne * Ne * Ne + 8.0 * Ne * Ne * Ne / 3.0);
+            else
+            {
+                launch_trace_and_negate_c(z(P.get()), Ne, nw * nb, z(tr.get()), st);
+                launch_lu_logdet_c(z(P.get()), Ne, nw * nb, z(ld.get()), st);
+            }
+            launches += 2;
+            tr.download(tr_h.data(), comp * nw * nb, st);
+            ld.download(ld_h.data(), comp * nw * nb, st);
+            GB_CUDA(cudaStreamSynchronize(st));
+            for (int s = 0; s < nb; ++s)
+                for (int w = 0; w < nw; ++w)
+                {
+                    const size_t i = comp * (static_cast<size_t>(s) * nw + w);
+                    const cplx v(tr_h[i] + ld_h[i], gamma_only ? 0.0 : tr_h[i + 1] + ld_h[i + 1]);
+                    res.per_q[qs[s0 + s]] += v * tf.omega_w[w] * ibz_w[qs[s0 + s]] / (2.0 * M_PI);
+                }
+            ec_flops += nb * nw * comp * comp * (2.0 * Ne * Ne * Ne + 2.0 * Ne * Ne * Ne / 3.0);
         }
     };
-    int lu_fallback_q = 0;
+    std::vector<int> lu_q;  // the q of the LU form
     if (use_chol)
     {
         // every q's V = L L^H in one batched factorisation, M' = I - L^H chi0 L per q on the tensor
@@ -897,8 +900,7 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
                 const int q = q0 + s;
                 if (badv[s])
                 {
-                    ec_lu_q(q);
-                    ++lu_fallback_q;
+                    lu_q.push_back(q);
                     continue;
                 }
                 launch_assemble_chi0(chi0_e + static_cast<long long>(q) * e_tot_e, static_cast<long long>(nq) * e_tot_e,
@@ -921,7 +923,9 @@ RpaResult run_rpa_gpu(Dataset &ds, const LibrpaOptions &opts, const TimeFreqGrid
                                                  : (2.0 * 8.0 * Ne * Ne * Ne + 4.0 * Ne * static_cast<double>(Ne) * Ne / 3.0));
         }
     }
-    for (int q = qa; q < qe && !use_chol; ++q) ec_lu_q(q);
+    const int lu_fallback_q = static_cast<int>(lu_q.size());
+    for (int q = qa; q < qe && !use_chol; ++q) lu_q.push_back(q);
+    ec_lu(lu_q);
     ev_ec.stop(st);
     S.t_ec = ev_ec.total_ms() * 1e-3;
     S.ec_flops = ec_flops;

@@ -113,5 +113,8 @@ void launch_trace_and_negate_r(double *P, int N, int batch, double *trace, cudaS
 // In-place LU with partial pivoting (one CTA per matrix); logdet = sum log(+-u_ii).
 void launch_lu_logdet_c(cuDoubleComplex *M, int N, int batch, cuDoubleComplex *logdet, cudaStream_t st);
 void launch_lu_logdet_r(double *M, int N, int batch, double *logdet, cudaStream_t st);
+// Random matrices (kind 0: uniform, 1: of -1, 0 and 1, 2: with one NaN) through the cluster LU and the one-CTA
+// LU: the largest difference of their log-determinants, infinite where only one of them is NaN.
+double lu_selftest(int N, int batch, bool is_complex, int kind, int seed);
 
 } // namespace gb

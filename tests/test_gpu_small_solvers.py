@@ -1,6 +1,7 @@
 """Edges of the small dense solvers (needs a GB300): the Cholesky's 64-wide diagonal blocks (last block of
-1 to 64 rows) through the tensor-core Cholesky's self-test, and the Gauss-Jordan solve of W_c, whose
-columns go to the CTAs of a cluster four at a time, through the Gamma-point G0W0 against the oracle."""
+1 to 64 rows) through the tensor-core Cholesky's self-test; the Gauss-Jordan solve of W_c, whose
+columns go to the CTAs of a cluster four at a time, through the Gamma-point G0W0 against the oracle; and
+the LU of E_c, whose columns go the same way to clusters of 1 to 8 CTAs, against the form with one CTA."""
 import ctypes
 import math
 
@@ -43,3 +44,19 @@ def test_wc_solve_through_g0w0(nabf):
     want = np.asarray(ref["sigc_iw"][0]).reshape(got.shape)
     # FP64 throughout; the frequency-to-time weights of a 6-point window amplify rounding by up to 1e3
     assert np.abs(got - want).max() <= 1e-11 * max(1.0, np.abs(want).max())
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2], ids=["uniform", "ties", "not_a_number"])
+@pytest.mark.parametrize("N,batch,complex_", [
+    (1, 3, 0), (3, 16, 1), (4, 16, 0),          # fewer column groups than CTAs of the cluster
+    (32, 16, 1), (33, 16, 0), (70, 38, 1),      # whole groups, a last group of one and of two columns
+    (304, 2, 1), (320, 2, 1), (450, 2, 0),      # columns in shared memory, in global memory
+    (30, 39, 1), (31, 77, 0), (30, 153, 1),     # clusters of 4, 2 and 1
+    (120, 153, 1),                              # one CTA a matrix, in global memory
+])
+def test_lu_log_determinant(lib, N, batch, complex_, kind):
+    d = lib.librpa_gb300_selftest_lu(N, batch, complex_, kind, 3 + N)
+    assert not math.isnan(d), lib.librpa_get_last_error(None).decode()
+    # the same operations per element in the same order; the compiler may fuse them differently: N 2^-52 with
+    # the condition of a random matrix (below 1e4 N)
+    assert d <= 1e-11 * N * N, d
