@@ -403,6 +403,7 @@ __global__ void __launch_bounds__(T1_THREADS, 1) k_t1_tc(const __grid_constant__
     }
     if (warp == 0) tmem_alloc(tmem_slot, T1_TMEM);
     __syncthreads();
+    pdl_trigger();  // T2 may take the SMs that this launch leaves idle
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
@@ -820,6 +821,7 @@ __global__ void __launch_bounds__(T2_THREADS) k_t2(const float4 *__restrict__ Xt
     float *tile = &buf[0][0][0][0];  // [T2_TILE][T2_TILE] of a part
     static_assert(sizeof(buf) >= sizeof(float) * T2_TILE * T2_TILE, "a part's tile fits the staging buffers");
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    pdl_wait();  // T1 has written chi0(R)
     if (nsplit > 1)
     {
         __syncthreads();
@@ -986,6 +988,7 @@ struct TcChi0::Impl
     T1Args t1_args(const double *G, double *chi0R) const;
     void autotune(const double *G, double *chi0R, cudaStream_t st);
     void launch_t1(const T1Args &a, cudaStream_t st);
+    void launch_t2(double *chi0R, cudaStream_t st);
 };
 
 namespace {
@@ -1207,9 +1210,39 @@ void TcChi0::Impl::launch_t1(const T1Args &a, cudaStream_t st)
     GB_LAUNCH_CHECK();
 }
 
+void TcChi0::Impl::launch_t2(double *chi0R, cudaStream_t st)
+{
+    const int tiles = (g.max_nabf + T2_TILE - 1) / T2_TILE;
+    // parts of a tile's steps while the tiles leave SMs idle, up to the portable cluster size; by the
+    // tiles of all blocks, so that a screened call sums a block as the unscreened one does
+    const long long ctas = static_cast<long long>(pr.n_pairs) * g.n_c * tiles * tiles;
+    const unsigned nsplit = static_cast<unsigned>(std::max<long long>(1, std::min<long long>(8, n_sm / ctas)));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(n_groups, tiles * tiles, nsplit);
+    cfg.blockDim = dim3(T2_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = nsplit;
+    // T2 reads what T1 reads and waits for it only to add to chi0(R), so it starts when T1's last CTAs do:
+    // beside it where T1 has fewer CTAs than there are SMs, in T1's last wave otherwise.  Before, T1 and T2
+    // took turns: a call of 3 atoms at Gamma 5.87 -> 5.37 ms, chi0 of 4 at 3 x 3 x 1 k 6.30 -> 5.80 ms
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    GB_CUDA(cudaLaunchKernelEx(&cfg, k_t2, static_cast<const float4 *>(Xt.get()),
+                               static_cast<const long long *>(xoff.get()), n4, g, pr,
+                               static_cast<const T1Group *>(groups.get()), tiles, chi0R));
+}
+
 // Times every candidate count of K parts per tile on this contraction's own inputs, one warm and
-// one timed launch each, and keeps the fastest.  The candidates write chi0R; the caller's own launch
-// after the tuning overwrites it (zeroing it first when tiles are split).
+// one timed launch each, and keeps the fastest.  T1 and T2 are timed together, since T2 runs beside T1 on
+// the SMs that T1 leaves: with T1 alone the tuner took 16 parts at 2 atoms of 13/40 on 2 x 2 x 2 k, which
+// left T2 24 SMs and cost 5% of the call.  The candidates write chi0R; the caller's own launch after the
+// tuning overwrites it (zeroing it first when tiles are split).
 void TcChi0::Impl::autotune(const double *G, double *chi0R, cudaStream_t st)
 {
     const T1Args a = t1_args(G, chi0R);
@@ -1227,8 +1260,10 @@ void TcChi0::Impl::autotune(const double *G, double *chi0R, cudaStream_t st)
         build_work(nullptr, st);
         if (n_work == 0) continue;
         launch_t1(a, st);
+        launch_t2(chi0R, st);
         GB_CUDA(cudaEventRecord(e0, st));
         launch_t1(a, st);
+        launch_t2(chi0R, st);
         GB_CUDA(cudaEventRecord(e1, st));
         GB_CUDA(cudaEventSynchronize(e1));
         float ms = 0.0f;
@@ -1377,25 +1412,7 @@ int TcChi0::contract(const double *G, double *chi0R, const unsigned char *active
         if (m.n_work > 0)
         {
             m.launch_t1(a, st);
-            const int tiles = (g.max_nabf + T2_TILE - 1) / T2_TILE;
-            // parts of a tile's steps while the tiles leave SMs idle, up to the portable cluster size; by the
-            // tiles of all blocks, so that a screened call sums a block as the unscreened one does
-            const long long ctas = static_cast<long long>(m.pr.n_pairs) * g.n_c * tiles * tiles;
-            const unsigned nsplit = static_cast<unsigned>(std::max<long long>(1, std::min<long long>(8, m.n_sm / ctas)));
-            cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3(m.n_groups, tiles * tiles, nsplit);
-            cfg.blockDim = dim3(T2_THREADS);
-            cfg.stream = st;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = 1;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = nsplit;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            GB_CUDA(cudaLaunchKernelEx(&cfg, k_t2, static_cast<const float4 *>(m.Xt.get()),
-                                       static_cast<const long long *>(m.xoff.get()), m.n4, g, m.pr,
-                                       static_cast<const T1Group *>(m.groups.get()), tiles, chi0R));
+            m.launch_t2(chi0R, st);
             launches += 2;
         }
     }
