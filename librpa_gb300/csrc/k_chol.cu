@@ -98,81 +98,117 @@ __global__ void __launch_bounds__(256) k_chol_diag(T *__restrict__ Aall, int N, 
 // diagonal of L, and with INV form W = L11^-1 (lower triangular, FP64) into Wb[b][64][64], so that the
 // panel becomes the product L21 = A21 W^T.
 //
-// Right-looking, the block in registers: thread 4 i + s holds the columns 4 k + s of row i.  Step p
-// scales column p, and with INV row p of what has been made of the identity, then subtracts their outer
-// product from the rows below; a row's columns up to p belong to the inverse and the later ones to A, so
-// one array of 16 holds both.  Bound by the pivots' chain and the FP64 pipe (1.6 FMAs per clock per SM):
-// the pivot takes one reciprocal square root instead of a square root and a division, two dependent
-// sequences of several hundred clocks each.  One GB300, a 64 x 64 block with its inverse: 216 -> 128 us.
+// Right-looking, the block in registers: thread (row i, s) holds the columns 8 k + s of row i.  With raw
+// column a_i of step p, pivot d and the inverse's unscaled row V_p (1 at p), the rows below take off
+// (a_i / d) times a_j to the right of p and (a_i / d) times V_pj up to p; a row's columns up to p belong
+// to the inverse and the later ones to A, so one array of 8 holds both.  Square roots wait until the end
+// (L_ip = a_i d_p^-1/2, W_p = d_p^-1/2 V_p): a step's chain is one barrier, a product, the update of the
+// next column and the next pivot's reciprocal.  Only whole warps skip work: the elements above the
+// diagonal are updated with whatever U holds and never read, so loads and FMAs stand without branches
+// between them.  A warp FMA occupies its scheduler's FP64 pipe for about 80 clocks and a warp of 4 rows
+// costs in proportion to the square of their index, so diag_rows deals the 16 warps' rows to the 4
+// schedulers evenly.  One GB300, a 64 x 64 block with its inverse: 216 us with the block in shared memory,
+// 128 with the roots in the chain and two barriers a step, 111 with a branch per element, now 80 (and 61 without the
+// inverse: the pivots' chain).
+constexpr int DIAG_THREADS = 512;
+
+// first of the 4 rows of a warp: warps w, w + 4, w + 8 and w + 12 share a scheduler
+__device__ inline int diag_rows(int warp) { return 4 * static_cast<int>(0x621075438BA9CDEFull >> (4 * warp) & 15); }
+
 template <bool INV>
-__global__ void __launch_bounds__(256) k_chol_diag64(double *__restrict__ Aall, int N, int k0, double *__restrict__ diag,
-                                                    int *__restrict__ bad, double *__restrict__ Wb)
+__global__ void __launch_bounds__(DIAG_THREADS) k_chol_diag64(double *__restrict__ Aall, int N, int k0,
+                                                             double *__restrict__ diag, int *__restrict__ bad,
+                                                             double *__restrict__ Wb)
 {
-    constexpr int NBT = OZAKI_NB;
-    static_assert(NBT == 64, "four threads a row, 16 columns each");
-    __shared__ double col[NBT], U[NBT], sinv;
+    constexpr int NBT = OZAKI_NB, KC = NBT / 8;
+    static_assert(NBT == 64, "eight threads a row, 8 columns each");
+    __shared__ double U[2][NBT], rinv[2], piv[NBT], raw[NBT][NBT + 1];
     const int b = blockIdx.x, nb = min(NBT, N - k0);
-    const int i = static_cast<int>(threadIdx.x) / 4, s = threadIdx.x % 4;
-    double *row = Aall + static_cast<long long>(b) * N * N + static_cast<long long>(k0 + i) * N + k0;
-    double v[16];
+    const int r0 = diag_rows(threadIdx.x / 32), lane = threadIdx.x % 32;
+    const int i = r0 + lane / 8, s = lane % 8;
+    double *A = Aall + static_cast<long long>(b) * N * N + static_cast<long long>(k0) * N + k0;
+    double v[KC];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) v[k] = i < nb && 4 * k + s <= i ? row[4 * k + s] : 0.0;
-#pragma unroll
-    for (int kp = 0; kp < 16; ++kp)
-#pragma unroll 1
-        for (int sp = 0; sp < 4; ++sp)
+    for (int k = 0; k < KC; ++k) v[k] = i < nb && 8 * k + s <= i ? A[static_cast<long long>(i) * N + 8 * k + s] : 0.0;
+    for (int t = threadIdx.x; t < 2 * NBT; t += DIAG_THREADS) U[t / NBT][t % NBT] = 0.0;
+    __syncthreads();
+    // column n and the pivot of step n; x is this thread's element of column n (s == n % 8)
+    auto hand_column = [&](int n, double &x) {
+        if (s != n % 8) return;
+        if (i > n && i < nb)
         {
-            const int p = 4 * kp + sp;
+            U[n & 1][i] = x;
+            raw[i][n] = x;
+            x = 0.0;
+        }
+        if (i == n)
+        {
+            if (!(x > 0.0)) bad[b] = 1;
+            const double d = fmax(x, 1e-300);
+            piv[n] = d;
+            rinv[n & 1] = 1.0 / d;
+            U[n & 1][n] = 1.0;
+            x = 1.0;
+        }
+    };
+    hand_column(0, v[0]);
+#pragma unroll
+    for (int kp = 0; kp < KC; ++kp)
+#pragma unroll 1
+        for (int sp = 0; sp < 8; ++sp)
+        {
+            const int p = 8 * kp + sp;
             if (p >= nb) break;
-            if (i == p && s == sp)
-            {
-                const double d = fmax(v[kp], 1e-300);
-                if (!(v[kp] > 0.0)) bad[b] = 1;
-                const double inv = rsqrt(d);
-                sinv = inv;
-                double l = d * inv;  // sqrt(d), corrected to its own rounding
-                l = fma(fma(-l, l, d), 0.5 * inv, l);
-                row[p] = l;
-                diag[static_cast<long long>(b) * N + k0 + p] = l;
-            }
             __syncthreads();
-            const double inv = sinv;
-            if (i > p && i < nb && s == sp)
+            if (r0 + 3 <= p) continue;  // the warp's rows are done
+            const double *u = U[p & 1] + s;
+            const double c = i > p ? u[i - s] * rinv[p & 1] : 0.0;
+            const int n = p + 1;
+            v[kp] = fma(-c, u[8 * kp], v[kp]);
+            if (kp + 1 < KC && 8 * (kp + 1) <= r0 + 3) v[kp + 1] = fma(-c, u[8 * (kp + 1)], v[kp + 1]);
+            if (n < nb)
             {
-                const double c = v[kp] * inv;
-                row[p] = c;
-                col[i] = c;
-                U[i] = c;
-                v[kp] = 0.0;
+                if (sp < 7)
+                    hand_column(n, v[kp]);
+                else if (kp + 1 < KC)
+                    hand_column(n, v[kp + 1]);
             }
-            if (INV && i == p)
+            if (INV)
+#pragma unroll
+                for (int k = 0; k < kp; ++k) v[k] = fma(-c, u[8 * k], v[k]);
+#pragma unroll
+            for (int k = kp + 2; k < KC; k += 2)
+                if (8 * k <= r0 + 3)
+                {
+                    v[k] = fma(-c, u[8 * k], v[k]);
+                    if (k + 1 < KC) v[k + 1] = fma(-c, u[8 * (k + 1)], v[k + 1]);
+                }
+            if (INV && i == n && n < nb)
             {
 #pragma unroll
                 for (int k = 0; k <= kp; ++k)
-                {
-                    const int j = 4 * k + s;
-                    if (j < p) v[k] *= inv;
-                    if (j == p) v[k] = inv;
-                    if (j <= p) U[j] = v[k];
-                }
-            }
-            __syncthreads();
-            if (i > p && i < nb)
-            {
-                const double c = col[i];
-#pragma unroll
-                for (int k = INV ? 0 : kp; k < 16; ++k)
-                {
-                    const int j = 4 * k + s;
-                    if (j <= i && (INV || j > p)) v[k] = fma(-c, U[j], v[k]);
-                }
+                    if (8 * k + s < n) U[n & 1][8 * k + s] = v[k];
             }
         }
+    __syncthreads();
+    if (threadIdx.x < nb)
+    {
+        const double d = piv[threadIdx.x], l = sqrt(d);
+        raw[threadIdx.x][threadIdx.x] = d;
+        diag[static_cast<long long>(b) * N + k0 + threadIdx.x] = l;
+        piv[threadIdx.x] = 1.0 / l;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < nb * NBT; t += DIAG_THREADS)
+    {
+        const int r = t / NBT, j = t % NBT;
+        if (j <= r) A[static_cast<long long>(r) * N + j] = raw[r][j] * piv[j];
+    }
     if constexpr (INV)
     {
         double *w = Wb + (static_cast<long long>(b) * NBT + i) * NBT;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) w[4 * k + s] = i < nb && 4 * k + s <= i ? v[k] : 0.0;
+        for (int k = 0; k < KC; ++k) w[8 * k + s] = i < nb && 8 * k + s <= i ? v[k] * piv[i] : 0.0;
     }
 }
 
@@ -347,13 +383,13 @@ int chol_batched_r_ozaki(double *A, int N, int batch, double *diag, int *bad, Oz
         const int rows_below = N - k0 - nb;
         if (rows_below == 0)
         {
-            k_chol_diag64<false><<<batch, 256, 0, st>>>(A, N, k0, diag, bad, nullptr);
+            k_chol_diag64<false><<<batch, DIAG_THREADS, 0, st>>>(A, N, k0, diag, bad, nullptr);
             GB_LAUNCH_CHECK();
             ++launches;
             continue;
         }
         // every panel with rows below it is a full 64-wide one (panels step by 64)
-        k_chol_diag64<true><<<batch, 256, 0, st>>>(A, N, k0, diag, bad, w.winv);
+        k_chol_diag64<true><<<batch, DIAG_THREADS, 0, st>>>(A, N, k0, diag, bad, w.winv);
         GB_LAUNCH_CHECK();
         launches += 1 + ozaki_panel_solve(A, N, batch, k0, w, st);
         launches += ozaki_trailing_update(A, N, batch, k0 + nb, k0, nb, w, st);

@@ -1228,7 +1228,7 @@ void TcChi0::Impl::launch_t2(double *chi0R, cudaStream_t st)
     at[0].val.clusterDim.z = nsplit;
     // T2 reads what T1 reads and waits for it only to add to chi0(R), so it starts when T1's last CTAs do:
     // beside it where T1 has fewer CTAs than there are SMs, in T1's last wave otherwise.  Before, T1 and T2
-    // took turns: a call of 3 atoms at Gamma 5.87 -> 5.37 ms, chi0 of 4 at 3 x 3 x 1 k 6.30 -> 5.80 ms
+    // took turns: a call of 3 atoms at Gamma 5.87 -> 5.31 ms, chi0 of 3 at 3 x 3 x 1 k 6.30 -> 5.73 ms
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
