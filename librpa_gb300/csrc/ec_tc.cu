@@ -446,12 +446,9 @@ int EcChol::stage_q(const void *L, const void *X, int slot, cudaStream_t st)
         // B^T of L and A = L^T are the same K-major matrix: row n = L(:, n)
         split_transpose_f64(Lr, N, N, N, static_cast<int>(m.kpad), bl, st);
         split_transpose_f64(Lr, N, N, N, static_cast<int>(m.kpad), al, st);
-        for (int w = 0; w < nw; ++w)
-        {
-            SplitBufs aw{3, {a1.p[0] + w * rowsA * m.kpad, a1.p[1] + w * rowsA * m.kpad, a1.p[2] + w * rowsA * m.kpad}};
-            split_rows_f64(Xr + w * nn, N, N, N, static_cast<int>(m.kpad), aw, st);
-        }
-        launches += 2 + nw;
+        // all frequencies in one launch: their matrices follow one another in X and in the operand
+        split_rows_f64(Xr, N, static_cast<long long>(nw) * N, N, static_cast<int>(m.kpad), a1, st);
+        launches += 3;
     }
     // T = chi0 L  (rowsA x N per w); L is lower triangular, so the K range of an output column
     // block n starts at n (at 2n with the complex path's interleaved K)

@@ -2,7 +2,7 @@
 //
 // Right-looking, panel width NB = 32, three launches per panel step for the whole batch:
 //   k_chol_diag  : one CTA per matrix factors the NB x NB diagonal block in shared memory;
-//   k_chol_panel : each CTA solves a 64-row slab of the panel below it, X L11^H = A21;
+//   k_chol_panel : each CTA solves a 32-row slab of the panel below it, X L11^H = A21;
 //   k_chol_update: lower-triangle trailing update A22 -= L21 L21^H in 32 x 32 tiles.
 // The real variant chol_batched_r_ozaki uses panels of 64 and does the trailing update on the
 // tensor cores with exact integer slices (k_chol_ozaki.cu).
@@ -212,55 +212,65 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_chol_diag64(double *__restrict
     }
 }
 
-// Panel solve X L11^H = A21 for a 64-row slab per CTA (L11 already factored in A).  Full
-// panels run right-looking with the row in registers (x[p] /= L_pp, then x[q] -= x[p] conj L_qp
-// for every q > p: independent updates instead of one serial sum per p) and the reciprocal
-// diagonal precomputed once per CTA.
-template <typename T, int NBT>
-__global__ void __launch_bounds__(64) k_chol_panel(T *__restrict__ Aall, int N, int k0)
+__device__ inline double cfms_conj(double c, double a, double b) { return fma(-a, b, c); }
+__device__ inline cuDoubleComplex cfms_conj(cuDoubleComplex c, cuDoubleComplex a, cuDoubleComplex b)
 {
+    // c - a * conj(b)
+    return make_cuDoubleComplex(fma(-a.y, b.y, fma(-a.x, b.x, c.x)), fma(a.x, b.y, fma(-a.y, b.x, c.y)));
+}
+__device__ inline double cshfl(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ inline cuDoubleComplex cshfl(cuDoubleComplex v, int src)
+{
+    return make_cuDoubleComplex(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+
+// Panel solve X L11^H = A21 below a full diagonal block (L11 already factored in A), 32 rows a CTA.
+// Right-looking, x[p] /= L_pp, then x[q] -= x[p] conj L_qp for every q > p.  Four threads hold a row,
+// columns 4 k + s, and pass x[p] on by a shuffle, so that a few rows already give all four schedulers'
+// FP64 pipes a warp; that pipe is the bound (a warp FMA takes about 80 clocks of it, 640 of them a warp
+// with complex entries).  The staged L11 has a zero diagonal, so the update takes whole quads of columns.
+// One GB300, the panels of eight complex 80 x 80 matrices: 122 us a launch with a thread per row, now 31.
+constexpr int PANEL_THREADS = 128, PANEL_ROWS = PANEL_THREADS / 4;
+
+template <typename T, int NBT>
+__global__ void __launch_bounds__(PANEL_THREADS) k_chol_panel(T *__restrict__ Aall, int N, int k0)
+{
+    static_assert(NBT % 4 == 0, "four threads share a row's columns");
+    constexpr int KC = NBT / 4;
     __shared__ T D[NBT][NBT + 1];
     __shared__ double invd[NBT];
-    const int b = blockIdx.y;
-    T *A = Aall + static_cast<long long>(b) * N * N;
-    const int nb = min(NBT, N - k0);
-    for (int t = threadIdx.x; t < nb * nb; t += blockDim.x)
+    T *A = Aall + static_cast<long long>(blockIdx.y) * N * N;
+    for (int t = threadIdx.x; t < NBT * NBT; t += PANEL_THREADS)
     {
-        const int i = t / nb, j = t % nb;
-        D[i][j] = j <= i ? A[static_cast<long long>(k0 + i) * N + k0 + j] : czero<T>();
+        const int i = t / NBT, j = t % NBT;
+        const T v = A[static_cast<long long>(k0 + i) * N + k0 + j];
+        D[i][j] = j < i ? v : czero<T>();
+        if (j == i) invd[i] = 1.0 / cre(v);
     }
     __syncthreads();
-    for (int p = threadIdx.x; p < nb; p += blockDim.x) invd[p] = 1.0 / cre(D[p][p]);
-    __syncthreads();
-    const int r = k0 + nb + blockIdx.x * 64 + threadIdx.x;
-    if (r >= N) return;
-    T *row = A + static_cast<long long>(r) * N + k0;
-    if (nb == NBT)
-    {
-        T x[NBT];
+    const int lane = threadIdx.x % 32, s = lane % 4;
+    const int r = k0 + NBT + static_cast<int>(blockIdx.x) * PANEL_ROWS + static_cast<int>(threadIdx.x) / 4;
+    if (r - lane / 4 >= N) return;  // the whole warp: its rows lie below the matrix
+    T *row = A + static_cast<long long>(min(r, N - 1)) * N + k0;
+    T x[KC];
 #pragma unroll
-        for (int p = 0; p < NBT; ++p) x[p] = row[p];
+    for (int k = 0; k < KC; ++k) x[k] = row[4 * k + s];
 #pragma unroll
-        for (int p = 0; p < NBT; ++p)
+    for (int kp = 0; kp < KC; ++kp)
+#pragma unroll
+        for (int sp = 0; sp < 4; ++sp)
         {
-            x[p] = cscale(x[p], invd[p]);
+            const int p = 4 * kp + sp;
+            if (s == sp) x[kp] = cscale(x[kp], invd[p]);
+            const T xp = cshfl(x[kp], (lane & ~3) | sp);
 #pragma unroll
-            for (int q = p + 1; q < NBT; ++q) x[q] = csub(x[q], cconjmul_acc(czero<T>(), x[p], D[q][p]));
+            for (int k = kp; k < KC; ++k) x[k] = cfms_conj(x[k], xp, D[4 * k + s][p]);
         }
+    if (r >= N) return;
 #pragma unroll
-        for (int p = 0; p < NBT; ++p) row[p] = x[p];
-        return;
-    }
-    T x[NBT];
-    for (int p = 0; p < nb; ++p) x[p] = row[p];
-    for (int p = 0; p < nb; ++p)
-    {
-        T s = x[p];
-        for (int q = 0; q < p; ++q) s = csub(s, cconjmul_acc(czero<T>(), x[q], D[p][q]));
-        x[p] = cscale(s, invd[p]);
-    }
-    for (int p = 0; p < nb; ++p) row[p] = x[p];
+    for (int k = 0; k < KC; ++k) row[4 * k + s] = x[k];
 }
+
 
 // Trailing update of the lower triangle, 32 x 32 tiles (ti >= tj), K = panel width.
 template <typename T>
@@ -348,8 +358,9 @@ int chol_impl(T *A, int N, int batch, double *diag, int *bad, cudaStream_t st)
         ++launches;
         if (rows_below > 0)
         {
-            dim3 gp((rows_below + 63) / 64, batch);
-            k_chol_panel<T, NB><<<gp, 64, 0, st>>>(A, N, k0);
+            // with rows below it the panel is a full one
+            dim3 gp((rows_below + PANEL_ROWS - 1) / PANEL_ROWS, batch);
+            k_chol_panel<T, NB><<<gp, PANEL_THREADS, 0, st>>>(A, N, k0);
             GB_LAUNCH_CHECK();
             const int ntile = (rows_below + 31) / 32;
             dim3 gu(ntile * (ntile + 1) / 2, batch);

@@ -1,7 +1,8 @@
 """Edges of the small dense solvers (needs a GB300): the Cholesky's 64-wide diagonal blocks (last block of
 1 to 64 rows) through the tensor-core Cholesky's self-test; the Gauss-Jordan solve of W_c, whose
 columns go to the CTAs of a cluster four at a time, through the Gamma-point G0W0 against the oracle; and
-the LU of E_c, whose columns go the same way to clusters of 1 to 8 CTAs, against the form with one CTA."""
+the LU of E_c, whose columns go the same way to clusters of 1 to 8 CTAs, against the form with one CTA, and
+the panels of the complex Cholesky, through E_c against the LU form."""
 import ctypes
 import math
 
@@ -10,7 +11,7 @@ import pytest
 
 import librpa_gb300 as L
 from conftest import oracle_input
-from librpa_gb300.synthetic import cluster_gamma
+from librpa_gb300.synthetic import cluster_gamma, small_periodic
 from oracle.gw_oracle import g0w0_gamma
 from oracle.rpa_oracle import Options as OOpts
 
@@ -60,3 +61,22 @@ def test_lu_log_determinant(lib, N, batch, complex_, kind):
     # the same operations per element in the same order; the compiler may fuse them differently: N 2^-52 with
     # the condition of a random matrix (below 1e4 N)
     assert d <= 1e-11 * N * N, d
+
+
+@pytest.mark.parametrize("nabf", [(16, 17), (31, 33), (32, 33), (48, 49), (64, 65)])
+def test_complex_cholesky_panels(nabf):
+    # rows below a 32-wide panel: 1, 32, 33, 65, 97 (a CTA takes 32)
+    s = small_periodic(2, [3, 2], list(nabf), (2, 1, 1), nocc=1, seed=12, nfreq=6)
+    perq = {}
+    for path in (L.EC_LU_FP64, L.EC_CHOL_FP64):
+        with L.Handler() as h:
+            L.load_system(h, s)
+            h.set_gb300_options(L.gb300_options(chi0_precision=L.CHI0_FP64, ec_path=path))
+            _, q = h.get_rpa_correlation_energy(L.Options(nfreq=6, tfgrids_type=L.Minimax, minimax_emin=s.minimax_emin,
+                                                          minimax_emax=s.minimax_emax), L.n_ibz(s))
+            perq[path] = np.asarray(q)
+            assert h.stats()["ec_lu_fallback_q"] == 0
+    # ln det and tr of N x N matrices near 1 with V of condition below 1e3: N 2^-52 1e3 absolute, times
+    # frequency weights of below 50 Ha in all over 2 pi
+    N = sum(nabf)
+    assert np.abs(perq[L.EC_LU_FP64] - perq[L.EC_CHOL_FP64]).max() <= 1e-11 * N
