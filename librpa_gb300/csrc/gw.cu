@@ -110,6 +110,7 @@ __global__ void __cluster_dims__(GJ_CL, 1, 1) __launch_bounds__(256)
     auto at = [&](int i, int j) -> double * {
         return j < N ? A + static_cast<size_t>(i) * N + j : B + static_cast<size_t>(i) * M + (j - N);
     };
+    cl.sync();  // every CTA runs: its shared memory may be written
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     for (int k = 0; k < N; ++k)
     {
