@@ -85,11 +85,16 @@ __global__ void k_one_minus(double *__restrict__ A, int N, int batch)
 // A cluster of GJ_CL CTAs per batch entry shares the columns of [A | B], 4 adjacent ones at a time in
 // turn, so that a CTA reads and writes its own columns only.  The owner of column k searches it for the
 // pivot and hands pivot and column to the others through distributed shared memory; then each CTA swaps,
-// scales and eliminates in its columns right of k.  Bound by the FP64 pipe of the CTAs (1.6 FMAs per clock
-// per SM) and, below N ~ 100, by the step's two hand-overs; with one CTA per entry, 16 of 152 SMs worked,
-// 3.80 ms for 16 entries of N = M = 102 (now 0.97).
+// scales and eliminates in its columns right of k.  STAGED: its columns stay in its shared memory, else they
+// are worked on in place.  Bound by the FP64 pipe of the CTAs (1.6 FMAs per clock per SM) and, below
+// N ~ 100, by a step's latencies.  16 entries of N = M = 102: 3.80 ms with one CTA per entry (16 of 152 SMs
+// at work), 0.97 with the cluster in global memory, now 0.40.
 constexpr int GJ_CL = 8;
 
+// columns of [A | B] that a CTA may hold
+__host__ __device__ constexpr int gj_width(int N, int M) { return 4 * (((N + M + 3) / 4 + GJ_CL - 1) / GJ_CL); }
+
+template <bool STAGED>
 __global__ void __cluster_dims__(GJ_CL, 1, 1) __launch_bounds__(256)
     k_gj_solve(double *__restrict__ Aall, double *__restrict__ Ball, int N, int M, int *__restrict__ bad)
 {
@@ -100,16 +105,24 @@ __global__ void __cluster_dims__(GJ_CL, 1, 1) __launch_bounds__(256)
     extern __shared__ double sm[];
     double *col = sm;          // [2][N]: column k before the elimination step, rows k and pivot swapped
     double *rowk = sm + 2 * N; // row k of this CTA's columns
-    __shared__ double rv[8];
+    __shared__ unsigned long long rv[8];
     __shared__ int ri[8], piv_of[2];
     // local column jl is column j of [A | B], in ascending order
     const int groups = (N + M + 3) / 4, mine = groups > r ? (groups - r + GJ_CL - 1) / GJ_CL : 0;
     int nl = 4 * mine;
     if (mine > 0 && (groups - 1) % GJ_CL == r) nl -= 4 * groups - (N + M);
-    auto column = [&](int jl) { return ((jl / 4) * GJ_CL + r) * 4 + jl % 4; };
-    auto at = [&](int i, int j) -> double * {
+    const int width = gj_width(N, M);
+    double *own = rowk + width;  // [N][width]
+    auto global = [&](int i, int jl) -> double * {
+        const int j = ((jl / 4) * GJ_CL + r) * 4 + jl % 4;
         return j < N ? A + static_cast<size_t>(i) * N + j : B + static_cast<size_t>(i) * M + (j - N);
     };
+    auto at = [&](int i, int jl) -> double * { return STAGED ? own + i * width + jl : global(i, jl); };
+    if (STAGED)
+    {
+        for (int t = threadIdx.x; t < N * nl; t += 256) *at(t / nl, t % nl) = *global(t / nl, t % nl);
+        __syncthreads();
+    }
     cl.sync();  // every CTA runs: its shared memory may be written
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     for (int k = 0; k < N; ++k)
@@ -117,12 +130,14 @@ __global__ void __cluster_dims__(GJ_CL, 1, 1) __launch_bounds__(256)
         const int buf = k & 1;
         if ((k / 4) % GJ_CL == r)
         {
-            // pivot: largest |A[i][k]|, i >= k, the first of equals
-            double best = -1.0;
+            const int kl = k / 4 / GJ_CL * 4 + k % 4;  // column k here
+            // pivot: largest |A[i][k]|, i >= k, the first of equals, by the bits of |x| (magnitude_key):
+            // comparisons of doubles would queue on the FP64 pipe
+            unsigned long long best = 0;
             int bi = k;
             for (int i = k + threadIdx.x; i < N; i += 256)
             {
-                const double v = fabs(*at(i, k));
+                const unsigned long long v = magnitude_key(*at(i, kl));
                 if (v > best)
                 {
                     best = v;
@@ -131,7 +146,7 @@ __global__ void __cluster_dims__(GJ_CL, 1, 1) __launch_bounds__(256)
             }
             for (int o = 16; o > 0; o >>= 1)
             {
-                const double v = __shfl_xor_sync(0xffffffffu, best, o);
+                const unsigned long long v = __shfl_xor_sync(0xffffffffu, best, o);
                 const int vi = __shfl_xor_sync(0xffffffffu, bi, o);
                 if (v > best || (v == best && vi < bi))
                 {
@@ -153,57 +168,71 @@ __global__ void __cluster_dims__(GJ_CL, 1, 1) __launch_bounds__(256)
                     best = rv[q];
                     bi = ri[q];
                 }
-            if (threadIdx.x == 0 && !(best > 0.0)) atomicExch(bad, 1);
+            if (threadIdx.x == 0 && best <= 1) atomicExch(bad, 1);  // 0, or nothing but NaN
             for (int t = threadIdx.x; t < N * GJ_CL; t += 256)
             {
                 const int q = t / N, i = t % N;
-                cl.map_shared_rank(col, q)[buf * N + i] = *at(i == k ? bi : i == bi ? k : i, k);
+                cl.map_shared_rank(col, q)[buf * N + i] = *at(i == k ? bi : i == bi ? k : i, kl);
             }
             if (threadIdx.x < GJ_CL) cl.map_shared_rank(piv_of, threadIdx.x)[buf] = bi;
         }
         cl.sync();
         const double *ck = col + buf * N;
         const int piv = piv_of[buf];
-        const double pv = ck[k];
-        const double inv = pv != 0.0 ? 1.0 / pv : 0.0;
         // this CTA's columns right of k
         const int gk = k / 4;
         const int jl0 = (gk > r ? (gk - r + GJ_CL - 1) / GJ_CL * 4 : 0) + (gk % GJ_CL == r ? k % 4 + 1 : 0);
         for (int jl = jl0 + threadIdx.x; jl < nl; jl += 256)
         {
-            const int j = column(jl);
-            double x = *at(k, j);
+            // formed here, by the warps that need it: a division is some ten operations of the FP64 pipe
+            const double pv = ck[k], inv = pv != 0.0 ? 1.0 / pv : 0.0;
+            double x = *at(k, jl);
             if (piv != k)
             {
-                const double y = *at(piv, j);
-                *at(piv, j) = x;
+                const double y = *at(piv, jl);
+                *at(piv, jl) = x;
                 x = y;
             }
             x *= inv;
-            *at(k, j) = x;
+            *at(k, jl) = x;
             rowk[jl] = x;
         }
         __syncthreads();
         const int na = nl - jl0;
-        for (long long t = threadIdx.x; t < static_cast<long long>(N) * na; t += 256)
+        for (int t = threadIdx.x; t < N * na; t += 256)
         {
-            const int i = static_cast<int>(t / na), jl = jl0 + static_cast<int>(t % na);
+            const int i = t / na, jl = jl0 + t % na;
             const double f = ck[i];
-            if (i == k || f == 0.0) continue;
-            *at(i, column(jl)) -= f * rowk[jl];
+            if (i == k || (__double_as_longlong(f) << 1) == 0) continue;  // f == 0, off the FP64 pipe
+            *at(i, jl) -= f * rowk[jl];
         }
         __syncthreads();
     }
+    if (STAGED)
+        for (int t = threadIdx.x; t < N * nl; t += 256)
+        {
+            const int i = t / nl, jl = t % nl;
+            if (((jl / 4) * GJ_CL + r) * 4 + jl % 4 >= N) *global(i, jl) = *at(i, jl);
+        }
     cl.sync();  // no CTA leaves while another may still write into it
 }
 
-size_t gj_smem(int N, int M) { return sizeof(double) * (2 * static_cast<size_t>(N) + (N + M) / GJ_CL + 8); }
+constexpr size_t GJ_SMEM_MAX = 200 * 1024;
+
+size_t gj_smem(int N, int M, bool staged)
+{
+    return sizeof(double) * (2 * static_cast<size_t>(N) + gj_width(N, M) * (1 + (staged ? static_cast<size_t>(N) : 0)));
+}
 
 void launch_gj_solve(double *A, double *B, int N, int M, int batch, int *bad, cudaStream_t st)
 {
     static PerDeviceOnce attr;
-    attr.run([] { GB_CUDA(cudaFuncSetAttribute(k_gj_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); });
-    k_gj_solve<<<batch * GJ_CL, 256, gj_smem(N, M), st>>>(A, B, N, M, bad);
+    attr.run([] {
+        GB_CUDA(cudaFuncSetAttribute(k_gj_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GJ_SMEM_MAX));
+        GB_CUDA(cudaFuncSetAttribute(k_gj_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GJ_SMEM_MAX));
+    });
+    const bool staged = gj_smem(N, M, true) <= GJ_SMEM_MAX;
+    (staged ? k_gj_solve<true> : k_gj_solve<false>)<<<batch * GJ_CL, 256, gj_smem(N, M, staged), st>>>(A, B, N, M, bad);
     GB_LAUNCH_CHECK();
 }
 

@@ -146,7 +146,7 @@ __device__ inline cuDoubleComplex tlogpm(cuDoubleComplex u)
 // in its shared memory, else in M; per element the operations are the same either way, in the same order.
 // The bound is the FP64 pipe, 1.6 FMAs per clock per SM, and below N ~ 100 the latency of a step (pivot
 // search, division, hand-over, a thin update).  With one CTA of 1024 threads a matrix, in global memory and
-// one q at a time, 16 of 152 SMs worked: 8 x 0.96 ms for 8 q of 16 complex 80 x 80 matrices; now 0.74 ms
+// one q at a time, 16 of 152 SMs worked: 8 x 0.96 ms for 8 q of 16 complex 80 x 80 matrices; now 0.48 ms
 // for the 128 together, on two CTAs each.
 constexpr int LU_THREADS = 256, LU_CL_MAX = 8, LU_SMEM_MAX = 200 * 1024;
 
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(LU_THREADS) k_lu_logdet(T *__restrict__ Mall, 
             own[i * width + jl] = M[static_cast<long long>(i) * N + column(jl)];
         }
     cl.sync();  // every CTA runs (its shared memory may be written) and has its columns
-    __shared__ double bval[LU_THREADS / 32];
+    __shared__ unsigned long long bval[LU_THREADS / 32];
     __shared__ int bidx[LU_THREADS / 32], piv_of[2];
     const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
     for (int k = 0; k < N; ++k)
@@ -188,16 +188,16 @@ __global__ void __launch_bounds__(LU_THREADS) k_lu_logdet(T *__restrict__ Mall, 
         {
             const int kl = gk / CL * 4 + k % 4;
             // pivot (largest magnitude, first index on ties; row k if no element compares)
-            double best = -1.0;
+            unsigned long long best = 0;  // magnitude_key: comparisons of doubles queue on the FP64 pipe
             int bi = N;
             for (int i = k + threadIdx.x; i < N; i += LU_THREADS)
             {
-                const double v = mag1(*at(i, kl));
+                const unsigned long long v = magnitude_key(mag1(*at(i, kl)));
                 if (v > best) { best = v; bi = i; }
             }
             for (int o = 16; o > 0; o >>= 1)
             {
-                const double v = __shfl_xor_sync(0xffffffffu, best, o);
+                const unsigned long long v = __shfl_xor_sync(0xffffffffu, best, o);
                 const int vi = __shfl_xor_sync(0xffffffffu, bi, o);
                 if (v > best || (v == best && vi < bi)) { best = v; bi = vi; }
             }

@@ -10,6 +10,15 @@
 
 namespace gb {
 
+#ifdef __CUDACC__
+// Whole number that orders as |x| does, 0 for NaN, 1 for zero.
+__device__ inline unsigned long long magnitude_key(double x)
+{
+    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(x)) & 0x7FFFFFFFFFFFFFFFull;
+    return b > 0x7FF0000000000000ull ? 0 : b + 1;
+}
+#endif
+
 // Small index tables describing atoms and BvK cells (device pointers).
 struct Geom
 {
