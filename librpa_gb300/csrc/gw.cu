@@ -822,10 +822,10 @@ __global__ void k_home_rows(const double *__restrict__ U, int N, int nao, int na
 // Partial products of the last step of the closed form, a short and wide output over a K axis (b, s)
 // that is N n_ao long:
 //   P[z][p][q] = sum_{k in part} Yw[d][b][p][s] U[b][s][q],   k = b n_ao + s, z = d nsplit + part.
-// Bound: the FP64 pipe (2 FMAs per clock per SM).  One CTA per output tile would run one SM or a few
-// for the whole product (2-atom fcc cell on 2x2x2 k: 16 CTAs with K = 133k, 0.12 s), so K is cut into
-// parts that fill the chip; the parts are summed in order by k_sum_parts, which keeps the result
-// independent of the schedule.  TM = 32 serves outputs of at most 32 rows without padding to 64.
+// Bound: the FP64 pipe (2 FMAs per clock per SM, 1.9 reached with the tiles' padding).  One CTA per output
+// tile would run one SM or a few for the whole product (2-atom fcc cell on 2x2x2 k: 16 CTAs with K = 133k,
+// 0.12 s for all rows; the home rows in parts 1.85 ms), so K is cut into parts that fill the chip; the
+// parts are summed in order by k_sum_parts, which keeps the result independent of the schedule.  TM = 32 serves outputs of at most 32 rows without padding to 64.
 constexpr int HN = 64, HK = 16;
 
 template <int TM>
