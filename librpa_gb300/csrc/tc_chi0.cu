@@ -1394,8 +1394,9 @@ int TcChi0::contract(const double *G, double *chi0R, const unsigned char *active
     int launches = 0;
     if (!m.t1_simt && !active && !m.tuned) m.autotune(G, chi0R, st);
     if (!m.t1_simt) m.build_work(active, st);
-    // K-part tiles add into chi0(R), so their rows start from zero
-    if (zero_first || (!m.t1_simt && m.has_split))
+    // K-part tiles add into chi0(R), so their rows start from zero; a list of blocks that adds to an earlier
+    // one finds its own rows zero and must leave the others alone
+    if (zero_first || (!m.t1_simt && !active && m.has_split))
         GB_CUDA(cudaMemsetAsync(chi0R, 0, sizeof(double) * static_cast<size_t>(m.pr.e_total) * g.n_c, st));
     if (m.t1_simt)
     {

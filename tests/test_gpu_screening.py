@@ -111,6 +111,26 @@ def test_learned_screening_skips_blocks_at_the_plain_result(cluster, lib):
     assert abs(ec_mlp - ec_plain) < 1e-10, (ec_mlp, ec_plain)
 
 
+@pytest.mark.parametrize("kparts", [1, 4, 16])
+def test_violated_audit_adds_the_missing_blocks(cluster, monkeypatch, kparts):
+    """A model that predicts nothing above the threshold: the audited share of the blocks is contracted
+    first, violates the audit, and the others are added to it, also where the tiles are cut into K parts
+    that add into chi0(R).  The call then equals the plain rule's up to the order of FP64 additions."""
+    monkeypatch.setenv("LIBRPA_GB300_T1_LAUNCH", f"wide:{kparts}")
+    s = cluster
+    h = _handler(s, chi0_precision=1, screen_mode=L.SCREEN_THRESHOLD, screen_threshold=THR)
+    ec_plain, _ = h.get_rpa_correlation_energy(_opts(s), 1)
+    params = np.zeros(mlp.NPARAM, np.float32)
+    norm = np.concatenate([np.zeros(mlp.IN), np.ones(mlp.IN), [-40.0, 1.0, 0.0]]).astype(np.float32)
+    assert h.lib.librpa_gb300_set_screening_model(h.h, _ptr(params), _ptr(norm)) == 0
+    h.set_gb300_options(L.gb300_options(chi0_precision=1, screen_mode=L.SCREEN_MLP, screen_threshold=THR,
+                                        audit_fraction=0.5, seed=5))
+    ec, _ = h.get_rpa_correlation_energy(_opts(s), 1)
+    st = h.stats()
+    assert st["screen_fallbacks"] > 0 and st["blocks_computed"] < st["blocks_total"]
+    assert abs(ec - ec_plain) < 1e-10, (ec, ec_plain)
+
+
 def test_learned_screening_transfers_across_mixed_species_cells(lib, capsys):
     """Mixed species (NAO/ABF 5/20, 13/60, 26/110, the shapes of the mixed-species workload): the
     MLP trains on block norms logged by the plain runs of three other small cells, pooled with
