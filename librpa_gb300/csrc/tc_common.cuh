@@ -84,18 +84,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity)
 }
 
 // The same for a wait that is long beside the work of the other warps on its scheduler: it sleeps NAP
-// nanoseconds between polls, and is bounded by the number of polls alone (reading %globaltimer costs
-// more than a short wait).
+// nanoseconds between polls and reads the clock, which costs more than a short wait, every 256 of them.
 template <uint32_t NAP>
-__device__ __forceinline__ bool mbar_wait_nap(uint64_t *bar, uint32_t parity)
+__device__ __forceinline__ bool mbar_wait_nap(uint64_t *bar, uint32_t parity, uint32_t limit_ms = kWaitLimitNs / 1000000)
 {
-    constexpr uint32_t kPolls = 1u << 24;
-    for (uint32_t i = 0; i < kPolls; ++i)
+    uint32_t end = 0;  // of the wait, in units of 2^20 ns (1.05 ms)
+    do
     {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (NAP > 0) __nanosleep(NAP);
-    }
-    return false;
+#pragma unroll 1
+        for (uint32_t i = 0; i < 256; ++i)
+        {
+            if (mbar_try_wait(bar, parity)) return true;
+            if (NAP > 0) __nanosleep(NAP);
+        }
+        const uint32_t now = static_cast<uint32_t>(globaltimer_ns() >> 20);
+        if (end == 0) end = now + limit_ms;
+        if (static_cast<int32_t>(now - end) > 0) return false;
+    } while (true);
 }
 
 // One lane of a converged warp.  Code that a whole warp runs with this around the issuing instructions

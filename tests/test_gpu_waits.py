@@ -1,0 +1,27 @@
+"""Waits of the tensor-core kernels that run out: a wait on an mbarrier that nothing arrives at gives up
+after its limit of wall time and returns (needs a GB300)."""
+import os
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = Path(__file__).resolve().parents[1]
+
+
+def _nvcc():
+    return os.environ.get("NVCC") or shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+
+
+def test_waits_end_at_their_limit(tmp_path):
+    exe = tmp_path / "wait_check"
+    subprocess.run([_nvcc(), "-gencode", "arch=compute_103a,code=sm_103a", "-O2", "-std=c++17", "-I",
+                    str(ROOT / "librpa_gb300" / "csrc"), str(ROOT / "tests" / "wait_check.cu"), "-o", str(exe)], check=True)
+    lines = subprocess.run([str(exe)], capture_output=True, text=True, check=True, timeout=60).stdout.split("\n")
+    got = [[float(x) for x in ln.split()] for ln in lines if ln]
+    assert [g[0] for g in got] == [0, 20, 100]
+    for _, done, ms in got:
+        # 200 units of 2^20 ns; a poll may be suspended for a while, and the clock is read every 256 of them
+        assert done == 0 and 200 <= ms <= 1000, got
