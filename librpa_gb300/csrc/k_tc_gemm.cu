@@ -105,8 +105,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
         fence_barrier_init();
     }
+    // where many launches share err, it is read after the last: those after one that gave up do nothing
     if (warp == 0) tmem_alloc(tmem_slot, 4 * BN);
-    __syncthreads();
+    if (__syncthreads_or(threadIdx.x == 32 && __ldca(err) != 0))
+    {
+        if (warp == 0) tmem_dealloc(*tmem_slot, 4 * BN);
+        return;
+    }
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     bool ok = true;

@@ -401,8 +401,14 @@ __global__ void __launch_bounds__(T1_THREADS, 1) k_t1_tc(const __grid_constant__
         }
         fence_barrier_init();
     }
+    // the host reads err after the last launch: the CTAs that start after a wait was given up do nothing, where
+    // each would run out its own limits
     if (warp == 0) tmem_alloc(tmem_slot, T1_TMEM);
-    __syncthreads();
+    if (__syncthreads_or(threadIdx.x == 32 && __ldcg(a.err) != 0))
+    {
+        if (warp == 0) tmem_dealloc(*tmem_slot, T1_TMEM);
+        return;
+    }
     pdl_trigger();  // T2 may take the SMs that this launch leaves idle
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
@@ -987,6 +993,7 @@ struct TcChi0::Impl
     std::string shape_key;
     T1Args t1_args(const double *G, double *chi0R) const;
     void autotune(const double *G, double *chi0R, cudaStream_t st);
+    void check(cudaStream_t st) const;
     void launch_t1(const T1Args &a, cudaStream_t st);
     void launch_t2(double *chi0R, cudaStream_t st);
 };
@@ -1272,6 +1279,7 @@ void TcChi0::Impl::autotune(const double *G, double *chi0R, cudaStream_t st)
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    check(st);  // launches that gave a wait up time nothing
     kparts = best.kparts;
     kparts_forced = true;
     all_active = false;
@@ -1420,10 +1428,12 @@ int TcChi0::contract(const double *G, double *chi0R, const unsigned char *active
     return launches;
 }
 
-void TcChi0::check(cudaStream_t st) const
+void TcChi0::check(cudaStream_t st) const { impl_->check(st); }
+
+void TcChi0::Impl::check(cudaStream_t st) const
 {
     int herr = 0;
-    impl_->err.download(&herr, 1, st);
+    err.download(&herr, 1, st);
     GB_CUDA(cudaStreamSynchronize(st));
     GB_REQUIRE(herr == 0, "tensor-core chi0 kernel reported wait timeout code " + std::to_string(herr));
 }

@@ -25,3 +25,13 @@ def test_waits_end_at_their_limit(tmp_path):
     for _, done, ms in got:
         # 200 units of 2^20 ns; a poll may be suspended for a while, and the clock is read every 256 of them
         assert done == 0 and 200 <= ms <= 1000, got
+
+
+def test_launches_after_one_that_gave_up_do_nothing(lib, tmp_path):
+    from librpa_gb300.build import ARCH, CFLAGS, PKG
+    exe = tmp_path / "t1_give_up_check"
+    subprocess.run([_nvcc(), *ARCH, *[f for f in CFLAGS if f not in ("-Xptxas", "-warn-spills")],
+                    str(ROOT / "tests" / "t1_give_up_check.cu"), "-o", str(exe), "-L", str(PKG), "-l:liblibrpa_gb300.so",
+                    "-Xlinker", "-rpath", "-Xlinker", str(PKG), "-ldl"], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout + out.stderr
