@@ -115,24 +115,6 @@ __device__ __forceinline__ void named_bar_sync(int id, int n)
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
-// Three-piece BF16 split of a pair of FP32 values (hi, mid, lo), each piece packed as bf16x2
-// (element 0 in the low half).  Each piece takes the top 8 bits of what is left of the 24, so the three
-// together are the value exactly.  By masks and byte permutes: a float to BF16 conversion instruction
-// costs several times theirs.
-__device__ __forceinline__ void split3_pair(float2 e, uint32_t &h, uint32_t &m, uint32_t &l)
-{
-    constexpr uint32_t top = 0xffff0000u;
-    const float2 neg1 = make_float2(-1.0f, -1.0f);
-    uint32_t x = __float_as_uint(e.x), y = __float_as_uint(e.y);
-    h = __byte_perm(x, y, 0x7632);
-    const float2 r1 = __ffma2_rn(make_float2(__uint_as_float(x & top), __uint_as_float(y & top)), neg1, e);
-    x = __float_as_uint(r1.x);
-    y = __float_as_uint(r1.y);
-    m = __byte_perm(x, y, 0x7632);
-    const float2 r2 = __ffma2_rn(make_float2(__uint_as_float(x & top), __uint_as_float(y & top)), neg1, r1);
-    l = __byte_perm(__float_as_uint(r2.x), __float_as_uint(r2.y), 0x7632);
-}
-
 // A = E in TMEM: D(tmem) (+)= A(tmem) * B(smem desc)^T, BF16 inputs, FP32 accumulate.  Row r of A is
 // TMEM lane r, each 32-bit column two consecutive K elements.
 __device__ __forceinline__ void mma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
