@@ -53,7 +53,7 @@ DeviceArena *current_arena();
 void *arena_take(DeviceArena *a, size_t bytes);
 void arena_give(DeviceArena *a, void *p);
 void release_idle_arenas();
-// cudaMalloc; where it fails, once more after what the arenas hold idle has gone back to the driver
+// cudaMalloc; where it fails, again after what the arenas hold unused has gone back to the driver
 void *device_malloc(size_t bytes);
 
 class ArenaScope
