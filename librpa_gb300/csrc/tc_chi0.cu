@@ -53,6 +53,7 @@ constexpr int T1_MAXA = 32;                        // max NAOs per atom
 constexpr int T1_CELLS = 32;                       // cells of a row group's shift table in shared memory
 constexpr int T1_INFO = 8;                         // ints kept of a row group: pair, cell, I, n_abf(I), n_ao(I)
 constexpr int T1_SMEM_MAX = 227 * 1024;
+constexpr long long T1_XSLAB = 2LL << 30;          // bytes of row-major X at a time; the contraction reads its re-ordered copy
 // Shared memory: nbs x NS B pieces of b_tile bytes | X ring | G blocks | barriers.  b_tile = NT_max * 128
 // rounded up to 1024; a G block holds, per 8 j, the 2 n_ao(I) rows q = (pass, i).
 
@@ -873,14 +874,14 @@ __global__ void k_gsT_split(const double *__restrict__ G, Geom g, long long kpad
 //   Xt[xoff[I] + (g4 t1_rows(a_I) + q) b_I + mu] = the 4 columns of X_b[(I, mu, i)], q = (pass, i),
 // pass 0 of X(-), pass 1 of X(+), zero rows past 2 a_I.  A warp of producers (32 consecutive rows mu)
 // then reads 512 contiguous bytes per q, where row-major X costs it 32 lines.  Grid: x = blocks of 8
-// groups, y = atoms times 32-row tiles of mu, z = blocks of T1_XD rows q; bound by HBM (X read and written once, 1% of the
-// contraction's time).
-__global__ void __launch_bounds__(256) k_x_layout(const float *__restrict__ X, long long xsign, Geom g, int n4, int ng4,
+// groups, y = atoms (from I0, whose first row is X's) times 32-row tiles of mu, z = blocks of T1_XD rows q;
+// bound by HBM (X read and written once, 1% of the contraction's time).
+__global__ void __launch_bounds__(256) k_x_layout(const float *__restrict__ X, long long xsign, Geom g, int I0, int n4, int ng4,
                                                   int mu_tiles, const long long *__restrict__ xoff,
                                                   float4 *__restrict__ Xt)
 {
     __shared__ float tile[T1_XD][32][33];
-    const int I = blockIdx.y / mu_tiles, mu0 = (blockIdx.y % mu_tiles) * 32;
+    const int I = I0 + blockIdx.y / mu_tiles, mu0 = (blockIdx.y % mu_tiles) * 32;
     const int aI = g.nao[I], bI = g.nabf[I], rows = t1_rows(aI), q0 = blockIdx.z * T1_XD;
     if (mu0 >= bI || q0 >= rows) return;
     const int c = threadIdx.x % 32, r0 = threadIdx.x / 32;
@@ -894,7 +895,7 @@ __global__ void __launch_bounds__(256) k_x_layout(const float *__restrict__ X, l
     {
         const int q = q0 + k;
         const bool lq = live && q < 2 * aI;
-        const float *src = X + (q < aI ? xsign : 0) + (g.rowc_off[I] + q % aI) * static_cast<long long>(g.n_sup) + col;
+        const float *src = X + (q < aI ? xsign : 0) + (g.rowc_off[I] - g.rowc_off[I0] + q % aI) * static_cast<long long>(g.n_sup) + col;
 #pragma unroll
         for (int r = 0; r < 32; r += 8)
             tile[k][r + r0][c] = lq && mu0 + r + r0 < bI ? src[static_cast<long long>(mu0 + r + r0) * aI * g.n_sup] : 0.0f;
@@ -951,6 +952,8 @@ struct TcChi0::Impl
     bool t1_simt = false;
     SplitStore csplit, gs;
     DevBuf<float> X, Gf, Cf;
+    std::vector<long long> row;  // first row of C of each atom, and their number
+    std::vector<int> slab;       // first atom of each slab of X, and the number of atoms
     DevBuf<float4> Xt;
     DevBuf<long long> xoff;
     DevBuf<int> err, cadd;
@@ -1012,13 +1015,15 @@ TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st)
     m.csplit.alloc(NS, static_cast<size_t>(g.rows_c) * m.kpad);
     split_rows_f64(C, nsup, g.rows_c, static_cast<int>(nsup), static_cast<int>(m.kpad), m.csplit.bufs(), st);
     m.gs.alloc(NS, 2ull * nsup * m.kpad);
-    m.X.alloc(2ull * g.rows_c * nsup);
     m.err.alloc(1);
     m.err.zero(st);
     // host copies of the small tables (Geom holds device pointers)
     std::vector<int> nao(g.n_at), nabf(g.n_at), cdiff(static_cast<size_t>(g.n_c) * g.n_c);
     GB_CUDA(cudaMemcpyAsync(nao.data(), g.nao, sizeof(int) * g.n_at, cudaMemcpyDeviceToHost, st));
     GB_CUDA(cudaMemcpyAsync(nabf.data(), g.nabf, sizeof(int) * g.n_at, cudaMemcpyDeviceToHost, st));
+    m.row.resize(g.n_at + 1);
+    GB_CUDA(cudaMemcpyAsync(m.row.data(), g.rowc_off, sizeof(long long) * g.n_at, cudaMemcpyDeviceToHost, st));
+    m.row[g.n_at] = g.rows_c;
     GB_CUDA(cudaMemcpyAsync(cdiff.data(), g.cdiff, sizeof(int) * cdiff.size(), cudaMemcpyDeviceToHost, st));
     std::vector<int> hI(pr.n_pairs), hJ(pr.n_pairs);
     GB_CUDA(cudaMemcpyAsync(hI.data(), pr.I, sizeof(int) * pr.n_pairs, cudaMemcpyDeviceToHost, st));
@@ -1032,12 +1037,23 @@ TcChi0::TcChi0(const Geom &g, const Pairs &pr, const double *C, cudaStream_t st)
     m.cadd.upload(cadd.data(), cadd.size(), st);
     if (m.t1_simt)
     {
+        m.X.alloc(2ull * g.rows_c * nsup);
         m.Cf.alloc(static_cast<size_t>(g.rows_c) * nsup);
         launch_d2f(C, m.Cf.get(), g.rows_c * nsup, st);
         m.Gf.alloc(2ull * g.n_c * g.n_ao * g.n_ao);
         return;
     }
     {
+        // X is formed for as many atoms at a time as T1_XSLAB bytes hold, at least one
+        long long most = 0;
+        m.slab.assign(1, 0);
+        for (int I = 1; I <= g.n_at; ++I)
+        {
+            if (I < g.n_at && 8 * nsup * (m.row[I + 1] - m.row[m.slab.back()]) <= T1_XSLAB) continue;
+            most = std::max(most, m.row[I] - m.row[m.slab.back()]);
+            m.slab.push_back(I);
+        }
+        m.X.alloc(2ull * most * nsup);
         std::vector<long long> xo(g.n_at);
         long long n = 0;
         for (int I = 0; I < g.n_at; ++I)
@@ -1365,15 +1381,22 @@ int TcChi0::prepare(const double *G, cudaStream_t st)
     const SplitBufs gb = m.gs.bufs();
     k_gsT_split<<<grid, 256, 0, st>>>(G, g, m.kpad, gb.p[0], gb.p[1], gb.p[2]);
     GB_LAUNCH_CHECK();
-    tc_gemm_split(m.csplit.mat(g.rows_c, m.kpad, 0), m.gs.mat(nsup, m.kpad, nsup * m.kpad), static_cast<int>(g.rows_c),
-                  static_cast<int>(nsup), static_cast<int>(nsup), 2, m.X.get(), nsup, g.rows_c * nsup, false,
-                  m.err.get(), st);
-    if (m.t1_simt) return 2;
     const int mu_tiles = (g.max_nabf + 31) / 32;
-    k_x_layout<<<dim3((m.ng4 + 7) / 8, g.n_at * mu_tiles, t1_rows(g.max_nao) / T1_XD), 256, 0, st>>>(m.X.get(), g.rows_c * nsup, g, m.n4, m.ng4,
-                                                                         mu_tiles, m.xoff.get(), m.Xt.get());
-    GB_LAUNCH_CHECK();
-    return 3;
+    const int n_slab = m.t1_simt ? 1 : static_cast<int>(m.slab.size()) - 1;
+    for (int k = 0; k < n_slab; ++k)
+    {
+        const int I0 = m.t1_simt ? 0 : m.slab[k], I1 = m.t1_simt ? g.n_at : m.slab[k + 1];
+        const long long rows = m.row[I1] - m.row[I0];
+        SplitMat C = m.csplit.mat(rows, m.kpad, 0);
+        for (int i = 0; i < NS; ++i) C.p[i] += m.row[I0] * m.kpad;
+        tc_gemm_split(C, m.gs.mat(nsup, m.kpad, nsup * m.kpad), static_cast<int>(rows), static_cast<int>(nsup),
+                      static_cast<int>(nsup), 2, m.X.get(), nsup, rows * nsup, false, m.err.get(), st);
+        if (m.t1_simt) return 2;
+        k_x_layout<<<dim3((m.ng4 + 7) / 8, (I1 - I0) * mu_tiles, t1_rows(g.max_nao) / T1_XD), 256, 0, st>>>(
+            m.X.get(), rows * nsup, g, I0, m.n4, m.ng4, mu_tiles, m.xoff.get(), m.Xt.get());
+        GB_LAUNCH_CHECK();
+    }
+    return 1 + 2 * n_slab;
 }
 
 int TcChi0::contract(const double *G, double *chi0R, const unsigned char *active, bool zero_first, cudaStream_t st)
