@@ -38,12 +38,12 @@ MEV_PER_ATOM_HA = 3.674932e-6  # 0.1 meV in Hartree
 PREC = {"bf16x3": 1, "fp32": 2, "fp64": 0}
 
 
-# DRAM bytes (read + write) of one per-(tau, spin) chi0 contraction launch set, from one ncu capture
-# per kernel on the same workload; None where no capture exists.
+# DRAM bytes (read + write) of one per-(tau, spin) chi0 contraction launch set, from an ncu capture on the
+# same workload on the default path; None where no capture exists.
 PROFILED_TRAFFIC = {
-    "fcc16_k333": {"bytes": 18.4119e9 + 0.0625e9 + 5.2037e9 + 0.3735e9,
-                   "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of k_t1_tc (tau_1) and the X "
-                             "k_tc_gemm (tau_0); k_t2 (1.4% of time) not captured"},
+    "fcc16_k333": {"bytes": 9.8436e9 + 0.0879e9 + 5.2981e9 + 0.3721e9 + 0.3743e9 + 0.3464e9 + 0.4213e9 + 0.0352e9,
+                   "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of k_t1_tc, the X k_tc_gemm, "
+                             "k_x_layout and k_t2 (tau_0)"},
 }
 
 def _peaks():

@@ -86,7 +86,7 @@ __global__ void k_one_minus(double *__restrict__ A, int N, int batch)
 // turn, so that a CTA reads and writes its own columns only.  The owner of column k searches it for the
 // pivot and hands pivot and column to the others through distributed shared memory; then each CTA swaps,
 // scales and eliminates in its columns right of k.  STAGED: its columns stay in its shared memory, else they
-// are worked on in place.  Bound by the FP64 pipe of the CTAs (1.6 FMAs per clock per SM) and, below
+// are worked on in place.  Bound by the FP64 pipe of the CTAs (1.68 FMAs per clock per SM) and, below
 // N ~ 100, by a step's latencies.  16 entries of N = M = 102: 3.80 ms with one CTA per entry (16 of 152 SMs
 // at work), 0.97 with the cluster in global memory, now 0.40.
 constexpr int GJ_CL = 8;
@@ -822,8 +822,8 @@ __global__ void k_home_rows(const double *__restrict__ U, int N, int nao, int na
 // Partial products of the last step of the closed form, a short and wide output over a K axis (b, s)
 // that is N n_ao long:
 //   P[z][p][q] = sum_{k in part} Yw[d][b][p][s] U[b][s][q],   k = b n_ao + s, z = d nsplit + part.
-// Bound: the FP64 pipe (2 FMAs per clock per SM, 1.9 reached with the tiles' padding).  One CTA per output
-// tile would run one SM or a few for the whole product (2-atom fcc cell on 2x2x2 k: 16 CTAs with K = 133k,
+// Bound: the FP64 pipe (1.68 FMAs per clock per SM in a loop of independent ones; 1.5 reached here, counting the
+// rows that fill a tile).  One CTA per output tile would run one SM or a few for the whole product (2-atom fcc cell on 2x2x2 k: 16 CTAs with K = 133k,
 // 0.12 s for all rows; the home rows in parts 1.85 ms), so K is cut into parts that fill the chip; the
 // parts are summed in order by k_sum_parts, which keeps the result independent of the schedule.  TM = 32 serves outputs of at most 32 rows without padding to 64.
 constexpr int HN = 64, HK = 16;

@@ -16,7 +16,7 @@
 // first CTA sums their tiles in order through distributed shared memory (the result does not depend on
 // the schedule).  Without the parts a 2-atom cell on 2x2x2 k ran on 24 of 152 SMs.
 //
-// Bound: FP64, its pipe (1.6 FMAs per clock per SM measured); FP32, the steps' latency in small cells and
+// Bound: FP64, its pipe (1.68 FMAs per clock per SM); FP32, the steps' latency in small cells and
 // shared-memory loads in large ones, which is why every operand is read as 4 columns at once.  One GB300,
 // per (tau, spin): FP64, 2 atoms of 13/40 on 2x2x2 k 4.67 -> 0.91 ms; FP32, 6 atoms of 36/140 and 13/60
 // 4.76 -> 0.75 ms.

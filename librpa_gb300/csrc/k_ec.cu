@@ -144,7 +144,7 @@ __device__ inline cuDoubleComplex tlogpm(cuDoubleComplex u)
 // pivot and hands the column, swapped and with the multipliers in place, to the others through distributed
 // shared memory; each CTA then swaps and eliminates in its columns right of k.  STAGED: a CTA's columns stay
 // in its shared memory, else in M; per element the operations are the same either way, in the same order.
-// The bound is the FP64 pipe, 1.6 FMAs per clock per SM, and below N ~ 100 the latency of a step (pivot
+// The bound is the FP64 pipe, 1.68 FMAs per clock per SM, and below N ~ 100 the latency of a step (pivot
 // search, division, hand-over, a thin update).  With one CTA of 1024 threads a matrix, in global memory and
 // one q at a time, 16 of 152 SMs worked: 8 x 0.96 ms for 8 q of 16 complex 80 x 80 matrices; now 0.48 ms
 // for the 128 together, on two CTAs each.

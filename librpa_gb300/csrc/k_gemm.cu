@@ -1,7 +1,7 @@
 // FP64 SIMT GEMMs (real and complex, row-major, batched by blockIdx.z).
 //
 // These serve the plain FP64 GPU path and the small complex products of the
-// G builder and E_c; on GB300 the FP64 pipe (~1.2 TFLOP/s) is the limit, so a
+// G builder and E_c; on GB300 the FP64 pipe (1.06 TFLOP/s) is the limit, so a
 // register-blocked 64x64 tile already sits on the FP64 roofline where its tiles fill the device.
 #include "kernels.h"
 #include "common.h"
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(256) k_gemm_real(int M, int N, int K, const T 
 }
 
 // The same product in 32 x 32 tiles of 128 threads, 4 x 2 outputs each, for shapes whose 64 x 64 tiles leave
-// SMs idle: the FP64 pipe of an SM does 1.6 FMAs a clock whatever it holds, so the number of SMs at work and
+// SMs idle: the FP64 pipe of an SM does 1.68 FMAs a clock whatever it holds, so the number of SMs at work and
 // the padding of the tiles set the time.  A thread's rows and columns beyond the matrix are left out, and
 // the next 16 of K are in flight during a block's FMAs.  Each element's sum runs over k in the same order
 // as in the larger tiles.  One GB300, 16 products of 102 x 102 x 102: 134 us in 64 x 64 tiles, now 56.

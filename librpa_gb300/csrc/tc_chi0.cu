@@ -202,13 +202,14 @@ __device__ __forceinline__ void t1_row(uint32_t xs, uint32_t ga, uint32_t gb, fl
 //   E[j][col] = sum_q G[q][j] X[q][col],   q = (pass, i),
 // then its 3-piece BF16 split, written to the warpgroup's A tile in TMEM half a stage (4 j) at a time.
 //
-// Bounds: 128 FP32 FMAs per clock per SM (the rows loop alone reaches 92), next to it the shared-memory
+// Bounds: 128 FP32 FMAs per clock per SM, next to it the shared-memory
 // path: a G value loaded serves the thread's 8 columns, an X value its j.  The two warpgroups work on
 // alternate chunks, so that the split and the hand-over of one run under the FMAs of the other.
 // Measured on one GB300 against two threads a row that wrote E to shared memory, with one drain warp
 // issuing everything, the whole chi0 stage: 128 atoms of 13/40 at Gamma 426 -> 289 ms, 48 atoms of 5/20,
-// 13/60 and 26/110 528 -> 112 ms, 16 atoms of 13/40 on 3x3x3 k 578 -> 394 ms.  What is left: two producer
-// warps per scheduler, 48 of 128 FMAs per clock over the kernel.
+// 13/60 and 26/110 528 -> 112 ms, 16 atoms of 13/40 on 3x3x3 k 578 -> 399 ms.  What is left: two producer
+// warps per scheduler, 46 of 128 FMAs of E per clock over the kernel (16 atoms), and 49% of the FMA pipe's
+// cycles with the split and the drain (ncu, 64 atoms of 13/40 at Gamma).
 template <int NJ, typename Fetch>
 __device__ __forceinline__ bool t1_unit(uint32_t xring, int &slot, const Fetch &fetch, uint32_t gs,
                                         int gq, int nq, int nhalf, uint32_t atile, uint64_t *full, uint64_t *empty, uint32_t &use,
@@ -1327,9 +1328,9 @@ void TcChi0::Impl::build_work(const unsigned char *active, cudaStream_t st)
     });
     // Every tile contracts the same K range, so the last, partial wave of CTAs leaves SMs idle:
     // its tiles are cut into K parts (added atomically into chi0(R)) when that shortens the
-    // makespan.  Launches of under 16 waves run every tile in T1_KPARTS K parts, finer units
-    // for the scheduler (measured: the 16-atom workload's 1155 tiles ran 6% faster as 4 parts,
-    // 8 parts no better; the 256-atom workload's 10k tiles gained nothing).
+    // makespan.  Every tile is cut into the count that the tuner timed; on a shape that it has not seen
+    // (a screened call), into T1_KPARTS where the launch has under 16 waves, finer units for the
+    // scheduler.
     has_split = false;
     {
         const std::vector<sched::KPart> plan =

@@ -103,14 +103,14 @@ __device__ __forceinline__ bool mbar_wait_nap(uint64_t *bar, uint32_t parity, ui
     } while (true);
 }
 
-// One lane of a converged warp.  Code that a whole warp runs with this around the issuing instructions
-// keeps their operands in uniform registers; under `lane == 0` each operand is moved there first.
 // Programmatic dependent launch.  The dependent grid may start once every CTA of this one has called
 // pdl_trigger or left; in the dependent, pdl_wait returns when the grids before it are complete and their
 // writes visible.  Without the launch attribute both do nothing.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// One lane of a converged warp.  Code that a whole warp runs with this around the issuing instructions
+// keeps their operands in uniform registers; under `lane == 0` each operand is moved there first.
 __device__ __forceinline__ bool elect_one()
 {
     uint32_t p;
