@@ -299,7 +299,6 @@ void launch_chi0_simt_rn(const T *Xp, const T *Xm, const T *Cm, const T *Gp, con
     const SimtShape sh = simt_shape<T>(g, RN);
     const bool g_smem = sizeof(T) * (sh.tiles + sh.gs) <= cap;
     const size_t smem = sizeof(T) * (sh.tiles + (g_smem ? sh.gs : 0));
-    GB_REQUIRE(smem <= cap, "atom NAO count too large for the SIMT chi0 kernel");
     // the cap once per device (calls of other shapes may run on other host threads)
     static PerDeviceOnce attr;
     attr.run([] {
@@ -335,6 +334,10 @@ template <typename T>
 void launch_chi0_simt(const T *Xp, const T *Xm, const T *Cm, const T *Gp, const T *Gm, const Geom &g,
                       const Pairs &pr, double *out, cudaStream_t st)
 {
+    // the sizes taken: a block of G and three operand tiles of 48 rows in shared memory (46 NAOs in FP64, 87 in
+    // FP32); these tiles would hold 49 and 99, at which a sum has 20 to 30% more terms
+    const size_t na = g.max_nao;
+    GB_REQUIRE(sizeof(T) * (na * na + 3 * TT * na * LC) <= 227 * 1024, "atom NAO count too large for the SIMT chi0 kernel");
     auto fits = [&](int rn) { return sizeof(T) * simt_shape<T>(g, rn).tiles <= 227 * 1024; };
     if (g.max_nabf > 96 && fits(9))
         launch_chi0_simt_rn<T, 9>(Xp, Xm, Cm, Gp, Gm, g, pr, out, st);
